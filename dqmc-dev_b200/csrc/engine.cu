@@ -572,53 +572,71 @@ __global__ void k_rotate_slices(int N, int L, int NB, int s, const double *src, 
 	}
 }
 
-// The delayed update runs as one CTA per chain with G in global memory
-// (k_update), or with G held in shared memory (k_update_cl, one CTA per
-// chain and spin in clusters of two) where one spin's G and panels fit
-// there.  Both do the same arithmetic in the same order.  The on-chip form
-// cuts the latency of a slice but holds a whole SM per CTA and pays a
-// cross-CTA exchange per accept.  Engines of real scalars with N >= 96 and
-// at most 64 chains take it: the 12 x 12 lattice at L = 120 ran 15% faster
-// from 1 to 64 chains (one chain 15.3 -> 17.7 chain-sweeps/s), 10 x 10 2%
-// faster, while 128 chains of 12 x 12 ran 5% slower and 4 x 4 and 8 x 8
-// 5-8% slower at every count.  DQMC_UPDATE=cluster or =global overrides
-// the rule (read when an engine is created, or a seam called).
-static bool update_cl_wanted(bool cplx, int N, int chains)
+// The delayed update runs as one CTA per chain with G in device memory
+// (k_update), or with G held in shared memory by a cluster of 2 P CTAs per
+// chain, P per spin (k_update_cl).  Both do the same arithmetic in the same
+// order.  The on-chip form shortens a slice but a chain then holds 2 P SMs, so
+// the rule goes by what fits at once and by what that gains.  Microseconds per
+// slice, device memory / P = 1 / 2 / 4 (real, then complex scalars):
+//   N = 16,    1 chain     16 /  17 /  17 /  18
+//   N = 64,    1 chain     44 /  39 /  38 /  39      103 /  80 /  74 /  73
+//   N = 64,   32 chains    47 /  41 /  40 / 100      112 /  87 /  81 / 198
+//   N = 64,  128 chains    48 /  73 / 137 / 296      114 / 162 / 286 / 602
+//   N = 100,   8 chains   108 /  75 /  67 /  63      290 /   - / 154 / 140
+//   N = 144,  32 chains   226 / 108 /  97 / 239
+//   N = 144, 256 chains   448 / 400 / 708 / 1422
+// More than one CTA per spin pays from N = 90 up (complex: 64), while the
+// clusters find room side by side: 2 P chains <= 128 CTAs for P = 2, half of
+// that for clusters of eight.  Beyond one wave of CTAs (74 chains) only the
+// larger lattices keep the on-chip form.  DQMC_UPDATE=cluster or =global
+// overrides the choice between the two forms (read when an engine is created,
+// or a seam called).  0: G in device memory, else P.
+template <typename T>
+static int update_split(int N, int kd, int chains)
 {
+	constexpr bool CX = is_cplx<T>::value;
 	const char *v = getenv("DQMC_UPDATE");
-	if (v && *v) return strcmp(v, "cluster") == 0;
-	return !cplx && N >= 96 && chains <= 64;
+	const bool cl = (v && *v) ? strcmp(v, "cluster") == 0
+	                          : N >= 25 && (chains <= 74 || N >= (CX ? 90 : 128));
+	if (!cl || N > 480) return 0;
+	const int p = (N >= 90 && chains <= 8) ? 4 : (N >= (CX ? 64 : 90) && chains <= 32) ? 2 : 1;
+	return update_cl_split<T>(N, kd, p);
 }
 
 template <typename T>
-static bool update_cl_fits(int N, int kd)
+static cudaError_t update_attr(int N, int kd, int ldp, int split)
 {
-	return N <= 480 && update_cl_smem_bytes<T>(N, kd) <= 226 * 1024;
+	if (split) return raise_smem(k_update_cl<T>, update_cl_smem_bytes<T>(N, split, kd));
+	const cudaError_t er = raise_smem(k_update<T>, update_smem_bytes<T>(N, kd, ldp));
+	return er != cudaSuccess ? er : raise_smem(k_update_big<T>, update_smem_bytes<T>(N, kd, ldp));
 }
 
+// the delayed update of a.nchain chains: on chip (split > 0), a cluster of
+// 2 split CTAs of cl_warps(N) warps and one look-ahead warp per chain; else one
+// CTA of update_warps(N) warps and one look-ahead warp per chain, in the launch
+// form sized for that CTA
 template <typename T>
-static cudaError_t update_attr(int N, int kd, size_t bytes, bool cl)
+static int launch_update(const UpdArgs<T> &a, cudaStream_t st, int split)
 {
-	if (cl) return raise_smem(k_update_cl<T>, update_cl_smem_bytes<T>(N, kd));
-	const cudaError_t e = raise_smem(k_update<T>, bytes);
-	return e != cudaSuccess ? e : raise_smem(k_update_big<T>, bytes);
-}
-
-// the delayed update of a.nchain chains: on chip (cl), two CTAs of
-// ceil(N/32) test warps and one look-ahead warp per chain; else one CTA of
-// 2 ceil(N/32) warps of tests and one look-ahead warp per chain, in the
-// launch form sized for that CTA
-template <typename T>
-static void launch_update(const UpdArgs<T> &a, size_t smem, cudaStream_t st, bool cl)
-{
-	if (cl) {
-		const int threads = (a.N + 31) / 32 * 32 + 32;
-		k_update_cl<T><<<2 * a.nchain, threads, update_cl_smem_bytes<T>(a.N, a.n_delay), st>>>(a);
-		return;
+	if (split) {
+		cudaLaunchConfig_t cfg = {};
+		cudaLaunchAttribute at = {};
+		at.id = cudaLaunchAttributeClusterDimension;
+		at.val.clusterDim.x = 2 * split;
+		at.val.clusterDim.y = at.val.clusterDim.z = 1;
+		cfg.gridDim = dim3(2 * split * a.nchain);
+		cfg.blockDim = dim3(cl_warps(a.N) * 32 + 32);
+		cfg.dynamicSmemBytes = update_cl_smem_bytes<T>(a.N, split, a.n_delay);
+		cfg.stream = st;
+		cfg.attrs = &at;
+		cfg.numAttrs = 1;
+		return cudaLaunchKernelEx(&cfg, k_update_cl<T>, a) == cudaSuccess ? 0 : DQMC_E_CUDA;
 	}
-	const int threads = 2 * ((a.N + 31) / 32 * 32) + 32;
+	const int threads = update_warps(a.N) * 32 + 32;
+	const size_t smem = update_smem_bytes<T>(a.N, a.n_delay, a.ldp);
 	if (threads <= 352) k_update<T><<<a.nchain, threads, smem, st>>>(a);
 	else k_update_big<T><<<a.nchain, threads, smem, st>>>(a);
+	return 0;
 }
 
 struct GroupBase {
@@ -682,7 +700,7 @@ struct Group : GroupBase, ProfHook {
 	int N, L, F, nmul;
 	int sweep = 0;
 	int kd = 0, ldp = 0;   // delayed-update flush period and panel ld
-	bool upd_cl = false;   // delayed update with G on chip (k_update_cl)
+	int upd_split = 0;     // CTAs per spin of the on-chip delayed update, 0: G in device memory
 	int eq_size = 0, ue_size = 0;
 	cudaStream_t st = nullptr;
 	std::map<int, cudaGraphExec_t> graphs;
@@ -953,11 +971,10 @@ struct Group : GroupBase, ProfHook {
 		}
 		if ((rc = toggle_maps(upv)) != 0) return rc;
 		// delayed-update panels: the file's n_delay unless shared memory is short
-		kd = p.n_delay < 1 ? 1 : p.n_delay;
 		ldp = (N + 15) / 16 * 16 + 4;
-		while (kd > 1 && update_smem_bytes<T>(N, kd, ldp) > 200 * 1024) kd /= 2;
-		upd_cl = update_cl_wanted(is_cplx<T>::value, N, engine_chains) && update_cl_fits<T>(N, kd);
-		CK(update_attr<T>(N, kd, update_smem_bytes<T>(N, kd, ldp), upd_cl));
+		kd = update_delay<T>(N, p.n_delay, ldp);
+		upd_split = update_split<T>(N, kd, engine_chains);
+		CK(update_attr<T>(N, kd, ldp, upd_split));
 		CK(cudaDeviceSynchronize());
 		return 0;
 	}
@@ -1220,7 +1237,7 @@ struct Group : GroupBase, ProfHook {
 	// the draws of slice l for every chain, from the working RNG state
 	void draws(int l)
 	{
-		k_draws<<<(C + 63) / 64, 64, 0, st>>>(N, L, C, l, del.p, rng.p, rng_ckpt.p, hs.p, order.p,
+		k_draws<<<C, 32, draws_smem_bytes(N), st>>>(N, L, C, l, del.p, rng.p, rng_ckpt.p, hs.p, order.p,
 		                                      ubuf.p);
 		launch_count++;
 	}
@@ -1236,7 +1253,7 @@ struct Group : GroupBase, ProfHook {
 		// slice again (L = 1), whose fields this kernel is still changing
 		a.next_slice = (L == 1) ? -1 : (l + 1) % L;
 		prof_begin(1);
-		launch_update<T>(a, update_smem_bytes<T>(N, kd, ldp), st, upd_cl);
+		launch_update<T>(a, st, upd_split);
 		prof_end(PC_UPDATE, 0.0, 0.0);
 		launch_count++;
 		watchdog("k_update");
@@ -1779,7 +1796,9 @@ struct Group : GroupBase, ProfHook {
 		precs.clear();
 	}
 
-	bool update_on_chip() override { return upd_cl; }
+	// whether the choice between the update's two forms fell on k_update_cl:
+	// it is offered where one spin's G fits one SM
+	bool update_on_chip() override { return upd_split > 0 && update_cl_split<T>(N, kd, 1) == 1; }
 
 	int profile_grad(int which, double *out, int ncls, int *launches) override
 	{
@@ -2894,23 +2913,21 @@ static int seam_update(int batch, int N, int n_delay, const double *del, uint64_
 {
 	if (batch < 1 || N < 1 || N > 480 || n_delay < 1 || !del || !rng || !hs || !G || !phase)
 		return DQMC_E_ARG;
-	int kd = n_delay;
-	const int ldp = (N + 15) / 16 * 16 + 4;
-	while (kd > 1 && update_smem_bytes<T>(N, kd, ldp) > 200 * 1024) kd /= 2;
-	const bool cl = update_cl_wanted(is_cplx<T>::value, N, batch) && update_cl_fits<T>(N, kd);
-	CK(update_attr<T>(N, kd, update_smem_bytes<T>(N, kd, ldp), cl));
+	const int ldp = (N + 15) / 16 * 16 + 4, kd = update_delay<T>(N, n_delay, ldp);
+	const int split = update_split<T>(N, kd, batch);
+	CK(update_attr<T>(N, kd, ldp, split));
 	Scratch<T> sc;
 	uint64_t *ck = sc.template get<uint64_t>((size_t)batch * 17);
 	int *ord = sc.template get<int>((size_t)batch * 2 * N);
 	double *uu = sc.template get<double>((size_t)batch * 2 * N);
 	if (!ck || !ord || !uu) return DQMC_E_NOMEM;
-	k_draws<<<(batch + 63) / 64, 64, 0, st>>>(N, 1, batch, 0, del, rng, ck, hs, ord, uu);
+	k_draws<<<batch, 32, draws_smem_bytes(N), st>>>(N, 1, batch, 0, del, rng, ck, hs, ord, uu);
 	UpdArgs<T> a;
 	memset(&a, 0, sizeof(a));
 	a.N = N; a.L = 1; a.n_delay = kd; a.nchain = batch; a.slice = 0; a.ldp = ldp;
 	a.del = del; a.rng = rng; a.rng_ckpt = ck; a.hs = hs; a.G = (T *)G; a.phase = (T *)phase;
 	a.order = ord; a.u = uu; a.next_slice = -1;
-	launch_update<T>(a, update_smem_bytes<T>(N, kd, ldp), st, cl);
+	launch_update<T>(a, st, split);
 	CK(cudaGetLastError());
 	CK(cudaStreamSynchronize(st));
 	return 0;

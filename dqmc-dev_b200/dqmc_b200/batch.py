@@ -19,9 +19,9 @@ files' value.  `autotune` also times every group of 32 chains or more in
 1, 2, 4 and 8 lanes (sub-batches whose launches overlap) and keeps the
 fastest, and for each lattice size it times the delayed update's two forms
 on the first group of that size: G in device memory with one CTA per chain
-and 8-column flush tiles per warp (k_update), or G on chip in a cluster of
-two CTAs per chain, one per spin (k_update_cl, where one spin's G and panels
-fit in shared memory).  Neither lanes nor the update form change results.
+(k_update), or G on chip in a cluster of CTAs per chain (k_update_cl), where
+one spin's G and panels fit in one SM's shared memory; larger lattices keep
+the engine's rule.  Neither lanes nor the update form change results.
 """
 from __future__ import annotations
 
@@ -72,8 +72,9 @@ def time_sweep(sims: list[SimData], n_delay: int | None, device: int = 0,
 
 
 def update_forms(sims: list[SimData], n_delay: int | None = None, device: int = 0) -> list[str]:
-    """The delayed-update forms these chains can take: "global" always,
-    "cluster" where the engine places one spin's G and panels on chip."""
+    """The delayed-update forms to choose from for these chains: "global"
+    always, "cluster" where one spin's G and panels fit in one SM's shared
+    memory."""
     e = Engine([sims[0].clone()], device=device, n_delay=n_delay, update="cluster")
     try:
         return ["global", "cluster"] if e.update_form == "cluster" else ["global"]
@@ -158,9 +159,11 @@ class RaggedBatch:
             for g, idx in enumerate(self.groups):
                 n = sims[idx[0]].N
                 if n not in self.update:
-                    self.update[n] = autotune_update([sims[i] for i in idx], device=device,
-                                                     n_delay=self.delay.get(n),
-                                                     lanes=self.lanes.get(g))
+                    group = [sims[i] for i in idx]
+                    # where there is no choice the engine's own rule stands
+                    self.update[n] = None if len(update_forms(group, self.delay.get(n), device)) == 1 \
+                        else autotune_update(group, device=device, n_delay=self.delay.get(n),
+                                             lanes=self.lanes.get(g))
         self.engines = [Engine([sims[i] for i in idx], device=device,
                                n_delay=self.delay.get(sims[idx[0]].N), lanes=self.lanes.get(g),
                                update=self.update.get(sims[idx[0]].N))

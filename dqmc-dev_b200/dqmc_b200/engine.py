@@ -183,10 +183,10 @@ class Engine:
         their own streams (else the engine's rule, or DQMC_LANES).  update
         selects the delayed update's form: "global" (G in device memory, one
         CTA per chain, k_update) or "cluster" (G on chip in a cluster of two
-        CTAs per chain, one per spin, k_update_cl, where one spin's G and
-        panels fit in shared memory; else "global"), else DQMC_UPDATE
-        decides, else the engine's rule (on chip for real scalars with
-        N >= 96 and at most 64 chains).  Results depend on neither lanes nor
+        to eight CTAs per chain, k_update_cl, where one spin's G and panels
+        fit the shared memory of four SMs; else "global"), else DQMC_UPDATE
+        decides, else the engine's rule (by N and the number of chains, see
+        dqmc_engine_update_on_chip).  Results depend on neither lanes nor
         update: every form does the same arithmetic in the same order."""
         if not sims:
             raise ValueError("no chains")
@@ -265,8 +265,9 @@ class Engine:
 
     @property
     def update_form(self) -> str:
-        """"cluster" when the delayed update holds G on chip (k_update_cl),
-        else "global" (dqmc_engine_update_on_chip)."""
+        """"cluster" when the delayed update holds G on chip (k_update_cl)
+        and one SM per spin would do, else "global"
+        (dqmc_engine_update_on_chip)."""
         r = self.lib.dqmc_engine_update_on_chip(self.h)
         _lib.check(min(r, 0), "dqmc_engine_update_on_chip")
         return "cluster" if r == 1 else "global"

@@ -170,8 +170,6 @@ struct EqWork {
 	T *G; long long g_stride;          // output
 	T *phi;                            // NB output phases
 	double *logdet;                    // NB, optional: log |det(I + C...C)|
-	const T *Pr; long long pr_stride;  // optional cache of the pair products
-	                                   // C_{(m+1)%F} C_m at Pr + b*pr_stride + m*N*N
 	unsigned *err;
 };
 
@@ -246,9 +244,7 @@ static int run_calc_eq_g(const EqWork<T> &w, int l0, cudaStream_t st, int *count
 	q.work = w.W; q.w_stride = NN;     // free while a QR runs
 	// factors in the first group: 1 + (F - 1) % group
 	const int first = 1 + (F - 1) % group;
-	if (first == 2 && w.Pr) {
-		q.X = w.Pr + (size_t)l0 * NN; q.x_stride = w.pr_stride;
-	} else if (first == 2) {
+	if (first == 2) {
 		eq_gemm(gargs<T>(N, N, N, NB, clu(l0 + 1), aCl, N, clu(l0), aCl, N, w.X, aI, N), st, count, ph, w.err);
 		q.X = w.X; q.x_stride = NN;
 	} else {
@@ -266,9 +262,6 @@ static int run_calc_eq_g(const EqWork<T> &w, int l0, cudaStream_t st, int *count
 		const int next = (m + group) % F;
 		if (group == 1) {
 			eq_gemm(gargs<T>(N, N, N, NB, clu(m), aCl, N, w.Qm, aI, N, w.X, aI, N), st, count, ph, w.err);
-		} else if (w.Pr) {
-			eq_gemm(gargs<T>(N, N, N, NB, w.Pr + (size_t)m * NN, Addr{w.pr_stride, 0, 1}, N, w.Qm, aI, N,
-			                 w.X, aI, N), st, count, ph, w.err);
 		} else {
 			eq_gemm(gargs<T>(N, N, N, NB, clu(m + 1), aCl, N, clu(m), aCl, N, w.W, aI, N), st, count, ph, w.err);
 			eq_gemm(gargs<T>(N, N, N, NB, w.W, aI, N, w.Qm, aI, N, w.X, aI, N), st, count, ph, w.err);
@@ -746,6 +739,8 @@ struct Group : GroupBase, ProfHook {
 	DevBuf<double> ubuf;
 	bool need_draws = true;
 	bool need_init = true;     // G must be recomputed from the fields before sweeping
+	// (Qm, dR, Tm / Tm2, qdet carry the left product from recalculation to
+	// recalculation within a sweep)
 	DevBuf<T> phase, G, Cl, Qm, Tm, Tm2, Rs, X, W, Gh, acc_eq, acc_ue, phi, qdet;
 	DevBuf<T> Sg;                  // gradient sums, allocated by the first logdet_grad
 	struct ObsWork {               // observable-gradient work, allocated by the first obs_grad
@@ -773,7 +768,12 @@ struct Group : GroupBase, ProfHook {
 			for (auto *x : d) x->release();
 		}
 	} ok;
-	DevBuf<T> Pr;                  // pair products C_{(m+1)%F} C_m, F >= 2
+	// The stack of a sweep: for f = 1 .. F-1 the decomposition of the clusters
+	// still to come, C_{F-1} ... C_f = T_f^H D_f Q_f^H, per f and item (f - 1
+	// first), built at the sweep's start from the last sweep's clusters
+	DevBuf<T> QL, TL, qdL;
+	DevBuf<double> dL;
+	bool stack = false;
 	DevBuf<double> dR, ldet;       // UDT scales; log |det(I + B...B)| per item
 	DevBuf<int> pvt;
 	DevBuf<unsigned> err;
@@ -793,13 +793,16 @@ struct Group : GroupBase, ProfHook {
 	bool check_acc = false;
 	DevBuf<T> Bacc, Gacc, phacc;       // [item][L] factors, [item] G and phase
 	DevBuf<double> ldacc;              // [item] log |det| of that recalculation
+	DevBuf<T> wacc[7];                 // its work: the sweep's own holds the product so far
+	DevBuf<double> dRacc;
+	DevBuf<int> pvacc;
 
 	~Group() override
 	{
 		for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
 		if (jev) cudaEventDestroy(jev);
 		DevBuf<T> *tb[] = {&expK, &iexpK, &ehK, &iehK, &peu, &ped, &phase, &G, &Cl, &Qm, &Tm,
-		                   &Tm2, &Rs, &X, &W, &Gh, &acc_eq, &acc_ue, &phi, &qdet, &Sg, &Pr,
+		                   &Tm2, &Rs, &X, &W, &Gh, &acc_eq, &acc_ue, &phi, &qdet, &Sg, &QL, &TL, &qdL,
 		                   &ppu, &ppd, &ppru, &pprd, &gs_eq, &gs_ue};
 		for (auto *b : tb) b->release();
 		DevBuf<int> *ib[] = {&i_off, &i_idx, &ij_off, &ij_idx, &bb_off, &bb_idx, &bonds, &hs,
@@ -812,6 +815,9 @@ struct Group : GroupBase, ProfHook {
 		ok.release();
 		Gw.release(); dmax.release(); dsum.release(); dcount.release();
 		Bacc.release(); Gacc.release(); phacc.release(); ldacc.release();
+		for (auto &b : wacc) b.release();
+		dRacc.release(); pvacc.release();
+		dL.release();
 		el.release(); del.release(); dv.release(); dvi.release(); dR.release(); ldet.release();
 		rng.release(); rng_ckpt.release(); order.release(); ubuf.release(); err.release();
 		ue.release();
@@ -926,7 +932,6 @@ struct Group : GroupBase, ProfHook {
 		rc |= Rs.alloc(NB * NN); rc |= X.alloc(NB * NN); rc |= W.alloc(NB * NN);
 		rc |= Gh.alloc(NB * NN); rc |= dR.alloc((size_t)NB * N); rc |= pvt.alloc((size_t)NB * N);
 		rc |= ldet.alloc(NB);
-		if (F >= 2) rc |= Pr.alloc((size_t)NB * F * NN);
 		rc |= err.alloc(1);
 		lay = acc_layout(p);
 		eq_size = (int)lay.eq_size;
@@ -935,6 +940,13 @@ struct Group : GroupBase, ProfHook {
 		if (ue_size) rc |= acc_ue.alloc((size_t)C * ue_size);
 		if (rc) return DQMC_E_NOMEM;
 		if (p.period_uneqlt > 0 && ue.alloc(N, L, F, NB)) return DQMC_E_NOMEM;
+		// without room for the stack every recalculation takes the whole chain
+		const size_t ns = (size_t)std::max(F - 1, 0) * NB;
+		stack = !(QL.alloc(ns * NN) | TL.alloc(ns * NN) | qdL.alloc(ns) | dL.alloc(ns * N));
+		if (!stack) {
+			QL.release(); TL.release(); qdL.release(); dL.release();
+			cudaGetLastError();
+		}
 		// parameter matrices, per spin
 		auto up2 = [&](DevBuf<T> &dst, const void *u, const void *d) {
 			cudaMemcpy(dst.p, u, sizeof(T) * NN, cudaMemcpyHostToDevice);
@@ -1070,9 +1082,15 @@ struct Group : GroupBase, ProfHook {
 			rc |= Gacc.alloc((size_t)NB * N * N);
 			rc |= phacc.alloc((size_t)NB);
 			rc |= ldacc.alloc((size_t)NB);
+			for (int k = 0; k < 6; k++) rc |= wacc[k].alloc((size_t)NB * N * N);
+			rc |= wacc[6].alloc((size_t)NB);
+			rc |= dRacc.alloc((size_t)NB * N);
+			rc |= pvacc.alloc((size_t)NB * N);
 			CK(cudaDeviceSynchronize());
 			if (rc) {
 				Bacc.release(); Gacc.release(); phacc.release(); ldacc.release();
+				for (auto &b : wacc) b.release();
+				dRacc.release(); pvacc.release();
 				return DQMC_E_NOMEM;
 			}
 		}
@@ -1094,8 +1112,8 @@ struct Group : GroupBase, ProfHook {
 	}
 
 	// G at slice l0 from the L single-slice factors, a QR after each
-	// (calc_eq_g(l0, N, L, 1, B, ...), dqmc.c:283-287), into Gacc; the
-	// cluster chain's scratch is free again once its G is done
+	// (calc_eq_g(l0, N, L, 1, B, ...), dqmc.c:283-287), into Gacc, in work
+	// matrices of its own
 	int calc_eq_g_acc(int l0)
 	{
 		const size_t NN = (size_t)N * N;
@@ -1105,7 +1123,8 @@ struct Group : GroupBase, ProfHook {
 		EqWork<T> w = eq_work();
 		w.F = L;
 		w.Cl = Bacc.p; w.cl_stride = (long long)L * NN;
-		w.Pr = nullptr;
+		w.Qm = wacc[0].p; w.Tm = wacc[1].p; w.Tm2 = wacc[2].p; w.Rs = wacc[3].p; w.X = wacc[4].p;
+		w.W = wacc[5].p; w.qdet = wacc[6].p; w.dR = dRacc.p; w.pvt = pvacc.p;
 		w.G = Gacc.p; w.g_stride = (long long)NN;
 		w.phi = phacc.p;
 		w.logdet = ldacc.p;
@@ -1193,16 +1212,6 @@ struct Group : GroupBase, ProfHook {
 		prof_end(0, fl, 3.0 * sizeof(T) * NN * NB * (nmul - 1));
 	}
 
-	// pair product m: C_{(m+1)%F} C_m of every item (the products that
-	// calc_eq_g's two-cluster groups start from)
-	void build_pair(int m)
-	{
-		const size_t NN = (size_t)N * N;
-		const Addr aC = per_item((long long)F * NN);
-		gemm(gargs<T>(N, N, N, NB, Cl.p + (size_t)((m + 1) % F) * NN, aC, N, Cl.p + (size_t)m * NN, aC, N,
-		              Pr.p + (size_t)m * NN, aC, N));
-	}
-
 	EqWork<T> eq_work()
 	{
 		EqWork<T> w;
@@ -1214,24 +1223,152 @@ struct Group : GroupBase, ProfHook {
 		w.G = G.p; w.g_stride = (long long)N * N;
 		w.phi = phi.p; w.err = err.p;
 		w.logdet = ldet.p;
-		w.Pr = Pr.p; w.pr_stride = (long long)F * N * N;
 		return w;
 	}
 
-	// G = (I + C_{l0-1} ... C_{l0})^-1 (cyclic), then the chain phases
+	// G = (I + C_{l0-1} ... C_{l0})^-1 (cyclic) from the whole chain of
+	// clusters, then the chain phases
 	int calc_eq_g(int l0)
 	{
-		// the only pair that calc_eq_g(l0) uses and whose clusters changed
-		// since it was formed is the one ending at cluster l0 - 1, the last
-		// rebuilt (its groups start at l0 (F even) or l0 + 1 (F odd) and
-		// step by two, always through (l0 - 2) mod F)
-		if (F >= 2) build_pair((l0 - 2 + F) % F);
 		int rc = run_calc_eq_g<T>(eq_work(), l0, st, &launch_count, profiling ? this : nullptr);
 		watchdog("calc_eq_g");
 		if (rc) return rc;
+		return combine_phase();
+	}
+
+	int combine_phase()
+	{
 		k_combine_phase<T><<<(C + 127) / 128, 128, 0, st>>>(C, phi.p, phase.p);
 		launch_count++;
 		return 0;
+	}
+
+	// ---------------------------------- recalculation with a stack
+	//
+	// After cluster f of a sweep is rebuilt, G needs the product of the
+	// rebuilt clusters on the left, C_f ... C_0, and of those still to come
+	// on the right, C_{F-1} ... C_{f+1}.  The first grows by one factor per
+	// recalculation (Qm, dR, Tm carry Q D T); the second runs through products
+	// that are all known at the sweep's start, where one pass over the
+	// clusters leaves the decomposition of each in the stack.  So a sweep
+	// takes 2 F - 1 factorisations where the whole chain at every
+	// recalculation (two clusters per factorisation, greens.c:69-208) takes
+	// F ceil(F / 2); at F = 12 that is 23 in place of 72.  Both sides are put
+	// together as
+	//   I + Q D T T_f^H D_f Q_f^H
+	//     = Q D_b [ D_b^-1 (Q^H Q_f) D_fb^-1 + D_s (T T_f^H) D_fs ] D_fb Q_f^H
+	// with the scales split into |d| > 1 (b) and the rest (s) on both sides,
+	// as the one-sided form splits D.  Against quad precision this G is no
+	// further off than the whole chain's (12x12, beta = 6: 5e-14 against
+	// 1.3e-13; 8x8, U = 6, beta = 8 from random fields: 7e-11 against 1e-8).
+
+	// one factorisation: X (or X^H) -> Q, diag, T; prev: the columns' scales
+	// and T so far (null: the first factor, column-pivoted)
+	int qdt(const T *Xin, long long xs, bool trans, const double *dprev, const T *Tprev, T *Q, double *d,
+	        T *Tout, T *qd)
+	{
+		const long long NN = (long long)N * N;
+		const double qfl = dense_flops<T>(N, NB), qby = 3.0 * sizeof(T) * NN * NB;
+		QrArgs<T> q;
+		memset(&q, 0, sizeof(q));
+		q.N = N; q.batch = NB; q.err = err.p;
+		q.X = Xin; q.x_stride = xs; q.trans = trans;
+		q.Q = Q; q.q_stride = NN;
+		q.dout = d; q.dout_stride = N;
+		q.qdet = qd;
+		q.pvt = pvt.p; q.p_stride = N;
+		q.work = W.p; q.w_stride = NN;
+		q.mode = dprev ? QR_PRESORT : QR_PIVOT;
+		if (dprev) {
+			q.dcol = dprev; q.d_stride = N;
+			q.Rs = Rs.p; q.r_stride = NN;
+		} else {
+			q.Tout = Tout; q.t_stride = NN;
+		}
+		prof_begin(0);
+		if (launch_qr<T>(q, st)) return DQMC_E_ARG;
+		prof_end(dprev ? PC_QR_PRESORT : PC_QR_PIVOT, qfl, qby);
+		launch_count++;
+		if (!dprev) return 0;
+		GemmArgs<T> g = gargs<T>(N, N, N, NB, Rs.p, per_item(NN), N, Tprev, per_item(NN), N, Tout, per_item(NN),
+		                         N, one<T>(), zero<T>(), GM_A_UPPER | GM_B_GATHER);
+		g.gidx = pvt.p;
+		g.aG = per_item(N);
+		gemm(g);
+		return 0;
+	}
+
+	// the decompositions of C_{F-1} ... C_f for f = F-1 .. 1
+	int build_stack()
+	{
+		const long long NN = (long long)N * N;
+		const Addr aC = per_item((long long)F * NN), aI = per_item(NN);
+		for (int f = F - 1; f >= 1; f--) {
+			const size_t o = (size_t)(f - 1) * NB, op = (size_t)f * NB;
+			const T *Cf = Cl.p + (size_t)f * NN;
+			int rc;
+			if (f == F - 1) {
+				rc = qdt(Cf, (long long)F * NN, true, nullptr, nullptr, QL.p + o * NN, dL.p + o * N, TL.p + o * NN,
+				         qdL.p + o);
+			} else {
+				gemm(gargs<T>(N, N, N, NB, Cf, aC, N, QL.p + op * NN, aI, N, X.p, aI, N, one<T>(), zero<T>(), GM_A_CT));
+				rc = qdt(X.p, NN, false, dL.p + op * N, TL.p + op * NN, QL.p + o * NN, dL.p + o * N, TL.p + o * NN,
+				         qdL.p + o);
+			}
+			if (rc) return rc;
+		}
+		watchdog("build_stack");
+		return 0;
+	}
+
+	// G after cluster f (called for f = 0, 1, ... F-1 in turn, after
+	// build_stack), then the chain phases
+	int recalc_g(int f)
+	{
+		if (!stack) return calc_eq_g((f + 1) % F);
+		const long long NN = (long long)N * N;
+		const Addr aC = per_item((long long)F * NN), aI = per_item(NN);
+		T *Tn = f % 2 ? Tm2.p : Tm.p, *To = f % 2 ? Tm.p : Tm2.p;   // T with and without cluster f
+		const T *Cf = Cl.p + (size_t)f * NN;
+		int rc;
+		if (f == 0) {
+			rc = qdt(Cf, (long long)F * NN, false, nullptr, nullptr, Qm.p, dR.p, Tn, qdet.p);
+		} else {
+			gemm(gargs<T>(N, N, N, NB, Cf, aC, N, Qm.p, aI, N, X.p, aI, N));
+			rc = qdt(X.p, NN, false, dR.p, To, Qm.p, dR.p, Tn, qdet.p);
+		}
+		if (rc) return rc;
+		const bool two = f + 1 < F;
+		const size_t o = (size_t)f * NB;       // f + 1 in the stack
+		RecArgs<T> ra;
+		memset(&ra, 0, sizeof(ra));
+		ra.N = N; ra.batch = NB;
+		ra.Q = Qm.p; ra.q_stride = NN;
+		ra.d = dR.p; ra.d_stride = N;
+		ra.qdet = qdet.p;
+		ra.phase = phi.p;
+		ra.work = W.p; ra.w_stride = NN;
+		ra.err = err.p;
+		ra.Tm = Tn; ra.t_stride = NN;
+		ra.G = G.p; ra.g_stride = NN;
+		if (two) {
+			gemm(gargs<T>(N, N, N, NB, Qm.p, aI, N, QL.p + o * NN, aI, N, X.p, aI, N, one<T>(), zero<T>(), GM_A_CT));
+			gemm(gargs<T>(N, N, N, NB, Tn, aI, N, TL.p + o * NN, aI, N, Rs.p, aI, N, one<T>(), zero<T>(), GM_B_CT));
+			ra.Wl = X.p; ra.wl_stride = NN;
+			ra.Tm = Rs.p;
+			ra.dl = dL.p + o * N; ra.dl_stride = N;
+			ra.qdetl = qdL.p + o;
+			ra.G = To;                           // free until the next cluster
+		} else {
+			ra.logdet = ldet.p;
+		}
+		prof_begin(0);
+		if (launch_rec<T>(ra, st)) return DQMC_E_ARG;
+		prof_end(PC_RECOMBINE, dense_flops<T>(N, NB), 3.0 * sizeof(T) * NN * NB);
+		launch_count++;
+		if (two) gemm(gargs<T>(N, N, N, NB, QL.p + o * NN, aI, N, To, aI, N, G.p, aI, N));
+		watchdog("recalc_g");
+		return combine_phase();
 	}
 
 	// the draws of slice l for every chain, from the working RNG state
@@ -1577,7 +1714,6 @@ struct Group : GroupBase, ProfHook {
 		const long long tot = (long long)C * 2 * L * N;
 		k_diag_all<<<grid_for(tot), 256, 0, st>>>(N, L, C, el.p, hs.p, dv.p, dvi.p);
 		for (int f = 0; f < F; f++) build_cluster(f);
-		for (int m = 0; F >= 2 && m < F; m++) build_pair(m);
 		int rc = calc_eq_g(0);
 		if (rc) return rc;
 		draws(0);
@@ -1597,6 +1733,10 @@ struct Group : GroupBase, ProfHook {
 	// queue one sweep of the given kind
 	int enqueue_sweep(bool meq, bool mue)
 	{
+		if (stack) {
+			const int rc = build_stack();
+			if (rc) return rc;
+		}
 		for (int l = 0; l < L; l++) {
 			update(l);
 			const int f = l / nmul;
@@ -1604,7 +1744,7 @@ struct Group : GroupBase, ProfHook {
 			if (recalc) {
 				if (check_g) wrap_into(l, Gw.p);
 				build_cluster(f);
-				int rc = calc_eq_g((f + 1) % F);
+				int rc = recalc_g(f);
 				if (rc) return rc;
 				if (check_g) {
 					k_gdrift<T><<<NB, 256, 0, st>>>(N, G.p, Gw.p, (long long)N * N, dmax.p, dsum.p,
@@ -1836,11 +1976,15 @@ struct Group : GroupBase, ProfHook {
 			CK(cudaDeviceSynchronize());   // its zeroing ran on the default stream
 		}
 		CK(cudaMemsetAsync(Sg.p, 0, sizeof(T) * NB * NN, st));
+		if (stack) {
+			const int rc = build_stack();
+			if (rc) return rc;
+		}
 		for (int l = 0; l < L; l++) {
 			k_grad_acc<T><<<grid_for((long long)NB * NN), 256, 0, st>>>(N, NB, L, l, G.p, dv.p, dvi.p, Sg.p);
 			launch_count++;
 			if ((l + 1) % nmul == 0) {
-				const int rc = calc_eq_g((l / nmul + 1) % F);
+				const int rc = recalc_g(l / nmul);
 				if (rc) return rc;
 			} else {
 				wrap(l);

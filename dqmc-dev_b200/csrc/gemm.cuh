@@ -18,6 +18,8 @@
 //                                        k-tiles left of the diagonal skipped)
 //   B_GATHER   B[k,c] = B[idx[k],c]     (row permutation P^T T)
 //   B_IDENT    B = I                    (C = alpha A + beta C)
+//   A_CT       A = S^H, S stored K x M   (Q^H X: the tile lands as B's do)
+//   B_CT       B = S^H, S stored N x K   (X T^H: the tile lands as A's do)
 // Tiles move global -> shared through a STAGES-deep ring, zero-filled
 // outside the matrix: in the TMA form one thread loads each stage's A and B
 // boxes with cp.async.bulk.tensor onto the stage's mbarrier (tensor maps over
@@ -41,6 +43,8 @@ enum : int {
 	GM_B_GATHER = 8,
 	GM_B_COLD = 16,
 	GM_B_IDENT = 32,
+	GM_A_CT = 64,
+	GM_B_CT = 128,
 };
 
 // off(b) = q * hi + (b % div) * lo with q = b / div, or q = tab[b / div]
@@ -104,15 +108,18 @@ __device__ inline void cp_async_el<zd>(zd *smem, const zd *gmem, bool valid)
 	cp_async16(smem, gmem, valid);
 }
 
-template <typename T, int BM, int BN, int BK, int WM, int WN, int STAGES>
+template <typename T, int BM, int BN, int BK, int WM, int WN, int STAGES, int MODE>
 struct GemmCfg {
 	static constexpr bool CX = is_cplx<T>::value;
 	static constexpr int THREADS = WM * WN * 32;
+	static constexpr bool A_CT = (MODE & GM_A_CT) != 0, B_CT = (MODE & GM_B_CT) != 0;
 	// padded strides: fragment reads conflict-free for 8- and 16-byte elements
-	static constexpr int SA = BM + (CX ? 2 : 4);      // As[k][r]
-	static constexpr int SB = BK + (CX ? 2 : 4);      // Bs[c][k]
-	static constexpr int TILE_A = BK * SA;
-	static constexpr int TILE_B = BN * SB;
+	static constexpr int PAD = CX ? 2 : 4;
+	static constexpr int SA = (A_CT ? BK : BM) + PAD;   // As[k][r], A_CT: As[r][k]
+	static constexpr int SB = (B_CT ? BN : BK) + PAD;   // Bs[c][k], B_CT: Bs[k][c]
+	static constexpr int NA = A_CT ? BM : BK, NBOX = B_CT ? BK : BN;   // strides per tile
+	static constexpr int TILE_A = NA * SA;
+	static constexpr int TILE_B = NBOX * SB;
 	static constexpr int STAGE = TILE_A + TILE_B;     // elements of T
 	static constexpr int KMAX = 512;                  // largest K of the scale vectors
 	static constexpr int RING_BYTES = STAGES * STAGE * (int)sizeof(T);
@@ -145,7 +152,7 @@ template <typename T, int BM, int BN, int BK, int WM, int WN, int STAGES, int MO
 __global__ void __launch_bounds__(WM *WN * 32)
 k_gemm(const __grid_constant__ GemmArgs<T> g)
 {
-	using Cfg = GemmCfg<T, BM, BN, BK, WM, WN, STAGES>;
+	using Cfg = GemmCfg<T, BM, BN, BK, WM, WN, STAGES, MODE>;
 	constexpr bool CX = Cfg::CX;
 	static_assert(!(TMA && (MODE & GM_B_GATHER)), "the row gather loads element by element");
 	extern __shared__ __align__(128) unsigned char gsm_raw[];
@@ -201,8 +208,10 @@ k_gemm(const __grid_constant__ GemmArgs<T> g)
 		T *Bs = As + Cfg::TILE_A;
 		const uint32_t mb = smem_u32(mbar + stage);
 		mbar_arrive_tx(mb, TX);
-		tma_load_4d(smem_u32(As), &g.tmA, E * m0, kt * BK, zA, wA, mb);
-		if (!(MODE & GM_B_IDENT)) tma_load_4d(smem_u32(Bs), &g.tmB, E * kt * BK, n0, zB, wB, mb);
+		if (Cfg::A_CT) tma_load_4d(smem_u32(As), &g.tmA, E * kt * BK, m0, zA, wA, mb);
+		else tma_load_4d(smem_u32(As), &g.tmA, E * m0, kt * BK, zA, wA, mb);
+		if (Cfg::B_CT) tma_load_4d(smem_u32(Bs), &g.tmB, E * n0, kt * BK, zB, wB, mb);
+		else if (!(MODE & GM_B_IDENT)) tma_load_4d(smem_u32(Bs), &g.tmB, E * kt * BK, n0, zB, wB, mb);
 	};
 	if constexpr (TMA) {
 		if (tid == 0) {
@@ -221,10 +230,11 @@ k_gemm(const __grid_constant__ GemmArgs<T> g)
 		for (int q = 0; q < Cfg::A_PER_T; q++) {
 			const int idx = tid + q * Cfg::THREADS;
 			if (idx < BM * BK) {
-				const int r = idx % BM, k = idx / BM;
+				const int r = Cfg::A_CT ? idx / BK : idx % BM, k = Cfg::A_CT ? idx % BK : idx / BM;
 				const int gr = m0 + r, gk = k0 + k;
 				const bool ok = gr < M && gk < K;
-				cp_async_el<T>(As + k * Cfg::SA + r, ok ? A + gr + (long long)gk * g.lda : A, ok);
+				const T *src = Cfg::A_CT ? A + gk + (long long)gr * g.lda : A + gr + (long long)gk * g.lda;
+				cp_async_el<T>(As + (Cfg::A_CT ? r * Cfg::SA + k : k * Cfg::SA + r), ok ? src : A, ok);
 			}
 		}
 		if (!(MODE & GM_B_IDENT)) {
@@ -232,12 +242,13 @@ k_gemm(const __grid_constant__ GemmArgs<T> g)
 			for (int q = 0; q < Cfg::B_PER_T; q++) {
 				const int idx = tid + q * Cfg::THREADS;
 				if (idx < BK * BN) {
-					const int k = idx % BK, c = idx / BK;
+					const int k = Cfg::B_CT ? idx / BN : idx % BK, c = Cfg::B_CT ? idx % BN : idx / BK;
 					const int gk = k0 + k, gc = n0 + c;
 					const bool ok = gk < K && gc < N;
 					int row = gk;
 					if (MODE & GM_B_GATHER) row = ok ? sgi[gk] : 0;
-					cp_async_el<T>(Bs + c * Cfg::SB + k, ok ? B + row + (long long)gc * g.ldb : B, ok);
+					const T *src = Cfg::B_CT ? B + gc + (long long)gk * g.ldb : B + row + (long long)gc * g.ldb;
+					cp_async_el<T>(Bs + (Cfg::B_CT ? k * Cfg::SB + c : c * Cfg::SB + k), ok ? src : B, ok);
 				}
 			}
 		}
@@ -302,7 +313,7 @@ k_gemm(const __grid_constant__ GemmArgs<T> g)
 #pragma unroll
 			for (int i = 0; i < Cfg::MT; i++) {
 				const int r = wm * Cfg::WTM + i * 8 + gq;
-				const T v = As[(kk + tq) * Cfg::SA + r];
+				const T v = Cfg::A_CT ? conjv(As[r * Cfg::SA + kk + tq]) : As[(kk + tq) * Cfg::SA + r];
 				double xr, xi;
 				split(v, xr, xi);
 				double sc = ka;
@@ -319,7 +330,7 @@ k_gemm(const __grid_constant__ GemmArgs<T> g)
 					xr = (gk == n0 + c) ? 1.0 : 0.0;
 					xi = 0.0;
 				} else {
-					const T v = Bs[c * Cfg::SB + kk + tq];
+					const T v = Cfg::B_CT ? conjv(Bs[(kk + tq) * Cfg::SB + c]) : Bs[c * Cfg::SB + kk + tq];
 					split(v, xr, xi);
 				}
 				double sc = kb;

@@ -12,7 +12,7 @@ namespace dq {
 template <typename T, int BM, int BN, int BK, int WM, int WN, int ST, int MODE, bool TMA>
 static int launch_gemm_form(const GemmArgs<T> &g, cudaStream_t st)
 {
-	using Cfg = GemmCfg<T, BM, BN, BK, WM, WN, ST>;
+	using Cfg = GemmCfg<T, BM, BN, BK, WM, WN, ST, MODE>;
 	if (raise_smem(k_gemm<T, BM, BN, BK, WM, WN, ST, MODE, TMA>, Cfg::SMEM_MAX, true) != cudaSuccess)
 		return DQMC_E_ARG;
 	// the grid's z extent is at most 65535: larger batches take several launches
@@ -32,7 +32,7 @@ static int launch_gemm_form(const GemmArgs<T> &g, cudaStream_t st)
 template <typename T, int BM, int BN, int BK, int WM, int WN, int ST, int MODE>
 static int launch_gemm_mode(const GemmArgs<T> &g, cudaStream_t st)
 {
-	using Cfg = GemmCfg<T, BM, BN, BK, WM, WN, ST>;
+	using Cfg = GemmCfg<T, BM, BN, BK, WM, WN, ST, MODE>;
 	if constexpr (!(MODE & GM_B_GATHER)) {
 		static const bool off = [] {
 			const char *e = getenv("DQMC_GEMM_TMA");
@@ -41,9 +41,11 @@ static int launch_gemm_mode(const GemmArgs<T> &g, cudaStream_t st)
 		constexpr int ED = is_cplx<T>::value ? 2 : 1;
 		GemmArgs<T> gt = g;
 		if (!off &&
-		    tma_map_operand(&gt.tmA, &gt.tzA, &gt.twA, g.A, ED, g.M, g.K, g.lda, g.aA, g.batch, Cfg::SA, BK) &&
+		    tma_map_operand(&gt.tmA, &gt.tzA, &gt.twA, g.A, ED, Cfg::A_CT ? g.K : g.M, Cfg::A_CT ? g.M : g.K, g.lda,
+		                    g.aA, g.batch, Cfg::SA, Cfg::NA) &&
 		    ((MODE & GM_B_IDENT) ||
-		     tma_map_operand(&gt.tmB, &gt.tzB, &gt.twB, g.B, ED, g.K, g.N, g.ldb, g.aB, g.batch, Cfg::SB, BN)))
+		     tma_map_operand(&gt.tmB, &gt.tzB, &gt.twB, g.B, ED, Cfg::B_CT ? g.N : g.K, Cfg::B_CT ? g.K : g.N, g.ldb,
+		                     g.aB, g.batch, Cfg::SB, Cfg::NBOX)))
 			return launch_gemm_form<T, BM, BN, BK, WM, WN, ST, MODE, true>(gt, st);
 	}
 	return launch_gemm_form<T, BM, BN, BK, WM, WN, ST, MODE, false>(g, st);
@@ -58,6 +60,8 @@ static int launch_gemm_cfg(const GemmArgs<T> &g, cudaStream_t st)
 	case GM_B_ROWD: return launch_gemm_mode<T, BM, BN, BK, WM, WN, ST, GM_B_ROWD>(g, st);
 	case GM_B_COLD: return launch_gemm_mode<T, BM, BN, BK, WM, WN, ST, GM_B_COLD>(g, st);
 	case GM_B_IDENT: return launch_gemm_mode<T, BM, BN, BK, WM, WN, ST, GM_B_IDENT>(g, st);
+	case GM_A_CT: return launch_gemm_mode<T, BM, BN, BK, WM, WN, ST, GM_A_CT>(g, st);
+	case GM_B_CT: return launch_gemm_mode<T, BM, BN, BK, WM, WN, ST, GM_B_CT>(g, st);
 	case GM_A_UPPER | GM_B_GATHER:
 		return launch_gemm_mode<T, BM, BN, BK, WM, WN, ST, GM_A_UPPER | GM_B_GATHER>(g, st);
 	default: return DQMC_E_ARG;

@@ -13,7 +13,8 @@
 //         diag(v) Q^H is elementwise), with the phase of det Q;
 // k_recb  G = (D_b^-1 Q^H + D_s T)^-1 D_b^-1 Q^H (greens.c:157-178) by LU
 //         with partial row pivoting and two triangular solves, plus the
-//         phase of det G (greens.c:194-207).
+//         phase of det G (greens.c:194-207); or the two-sided form of it for
+//         a product given as Q D T on its left and T_L^H D_L Q_L^H on its right.
 #pragma once
 
 #include "common.cuh"
@@ -26,6 +27,7 @@ template <typename T>
 struct QrArgs {
 	int N, batch, mode;
 	const T *X; long long x_stride;       // input matrices (ld N)
+	int trans;                            // PIVOT: factor X^H instead of X
 	const double *dcol; long long d_stride; // PRESORT: columns scaled by d on load
 	T *Q; long long q_stride;             // explicit Q out
 	T *Tout; long long t_stride;          // PIVOT: T = D^-1 R P^T
@@ -662,14 +664,19 @@ __global__ void __maxnreg__(96) k_qrp(QrArgs<T> a)
 	__shared__ int s_bi[NW];
 	bool nan_seen = false;
 	const T *X = a.X + (size_t)item * a.x_stride;
+	if (a.trans) {
+		for (int c = w; c < N; c += NW)
+			for (int r = lane; r < N; r += 32) A[c + (size_t)ld * r] = conjv(X[r + (size_t)N * c]);
+		__syncthreads();
+	}
 	{
 		double best = -1.0;
 		int bi = N;
 		for (int c = w; c < N; c += NW) {
 			double s = 0.0;
 			for (int r = lane; r < N; r += 32) {
-				const T v = X[r + (size_t)N * c];
-				A[r + (size_t)ld * c] = v;
+				const T v = a.trans ? A[r + (size_t)ld * c] : X[r + (size_t)N * c];
+				if (!a.trans) A[r + (size_t)ld * c] = v;
 				s += abs2(v);
 			}
 			s = sqrt(warp_sum(s));
@@ -801,6 +808,11 @@ struct RecArgs {
 	const T *Tm; long long t_stride;
 	const double *d; long long d_stride;
 	const T *qdet;
+	// two-sided form: the product is Q D T (T_L^H D_L Q_L^H); Wl = Q^H Q_L, Tm =
+	// T T_L^H, dl = D_L, and G receives D_Lb^-1 Z (the Q_L on its left follows)
+	const T *Wl; long long wl_stride;
+	const double *dl; long long dl_stride;
+	const T *qdetl;
 	T *G; long long g_stride;
 	T *phase;                 // per item: 1 / phase(det G)
 	double *logdet;           // per item, optional: log |det(I + B...B)| = -log |det G|
@@ -819,8 +831,9 @@ struct RecArgs {
 // of the solution is kept there in B layout (ys[64 t + 32 s + lane], k-step
 // s), each lane reading back only what it wrote, so the slab needs no
 // synchronisation; holding the tiles in registers instead spills.
+// osc: factors of the solution's rows on output (null: none).
 __device__ inline void recb_solve8(const double *M, int ld, const int *perm, const double *vsh,
-		const double *Q, double *G, int N, int c0, int lane, double *ys)
+		const double *Q, double *G, int N, int c0, int lane, double *ys, const double *osc)
 {
 	const int lr = lane & 3, lq = lane >> 2;
 	const int nt = (N + 7) / 8;
@@ -926,8 +939,9 @@ __device__ inline void recb_solve8(const double *M, int ld, const int *perm, con
 			}
 		}
 		if (r < N) {
-			if (cc < N) G[r + (size_t)N * cc] = x[0];
-			if (cc + 1 < N) G[r + (size_t)N * (cc + 1)] = x[1];
+			const double f = osc ? osc[r] : 1.0;
+			if (cc < N) G[r + (size_t)N * cc] = x[0] * f;
+			if (cc + 1 < N) G[r + (size_t)N * (cc + 1)] = x[1] * f;
 		}
 		c_to_b(x[0], x[1], yb(t, 0), yb(t, 1));
 	}
@@ -1000,9 +1014,25 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 		else { vsh[r] = 1.0; dss[r] = dr; }
 	}
 	__syncthreads();
-	for (int c = w; c < N; c += NW)
-		for (int r = lane; r < N; r += 32)
-			M[r + (size_t)ld * c] = conjv(Q[c + (size_t)N * r]) * vsh[r] + Tm[r + (size_t)N * c] * dss[r];
+	const double *osc = nullptr;
+	if (a.Wl) {
+		// D_b^-1 (Q^H Q_L) D_Lb^-1 + D_s (T T_L^H) D_Ls
+		const T *Wl = a.Wl + (size_t)item * a.wl_stride;
+		const double *dl = a.dl + (size_t)item * a.dl_stride;
+		for (int c = w; c < N; c += NW) {
+			const double x = dl[c], vl = fabs(x) > 1.0 ? 1.0 / x : 1.0, sl = fabs(x) > 1.0 ? 1.0 : x;
+			for (int r = lane; r < N; r += 32)
+				M[r + (size_t)ld * c] = Wl[r + (size_t)N * c] * (vsh[r] * vl) + Tm[r + (size_t)N * c] * (dss[r] * sl);
+		}
+		__syncthreads();
+		// D_s is spent: its place takes D_Lb^-1
+		for (int r = tid; r < N; r += blockDim.x) dss[r] = fabs(dl[r]) > 1.0 ? 1.0 / dl[r] : 1.0;
+		osc = dss;
+	} else {
+		for (int c = w; c < N; c += NW)
+			for (int r = lane; r < N; r += 32)
+				M[r + (size_t)ld * c] = conjv(Q[c + (size_t)N * r]) * vsh[r] + Tm[r + (size_t)N * c] * dss[r];
+	}
 	__syncthreads();
 
 	bool nan_seen = false, sing = false;
@@ -1116,7 +1146,7 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 		             + (size_t)64 * ((N + 7) / 8) * w;
 		for (int c0 = 8 * w; w < nws && c0 < N; c0 += 8 * nws)
 			recb_solve8((const double *)M, ld, perm, vsh, (const double *)Q, (double *)G, N, c0,
-			                     lane, ys);
+			                     lane, ys, osc);
 	}
 	for (int c0 = w * CB; !TC && c0 < N; c0 += NW * CB) {
 		T y[CB][RPL];
@@ -1187,7 +1217,7 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 #pragma unroll
 			for (int t = 0; t < RPL; t++) {
 				const int r = lane + 32 * t;
-				if (r < N) G[r + (size_t)N * c] = y[b][t];
+				if (r < N) G[r + (size_t)N * c] = osc ? y[b][t] * osc[r] : y[b][t];
 			}
 		}
 	}
@@ -1200,9 +1230,10 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 		for (int j = lane; j < N; j += 32) {
 			const T u = M[j + (size_t)ld * j];
 			ph = ph * phase_of(u);
-			neg ^= (vsh[j] < 0.0) ^ (ipiv[j] != j);
+			neg ^= (vsh[j] < 0.0) ^ (ipiv[j] != j) ^ (osc && osc[j] < 0.0);
 			// G = M^-1 diag(v) Q^H: log |det G| = sum log |v_j| - sum log |U_jj|
-			if (a.logdet) l += log(absv(u)) - log(fabs(vsh[j]));
+			// (two-sided: and sum log |v_L,j|)
+			if (a.logdet) l += log(absv(u)) - log(fabs(vsh[j])) - (osc ? log(fabs(osc[j])) : 0.0);
 		}
 #pragma unroll
 		for (int o = 16; o > 0; o >>= 1) {
@@ -1212,6 +1243,7 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 		}
 		if (lane == 0) {
 			if (a.qdet) ph = a.qdet[item] * ph;
+			if (osc && a.qdetl) ph = ph * conjv(a.qdetl[item]);
 			a.phase[item] = neg ? ph * -1.0 : ph;
 			if (a.logdet) a.logdet[item] = l;
 		}

@@ -76,7 +76,7 @@ int launch_qr_pivot(const QrArgs<T> &a, cudaStream_t st)
 template <typename T, int RPL, bool GM>
 static int launch_rec_rpl(const RecArgs<T> &a, cudaStream_t st)
 {
-	return launch_dense(k_recb<T, 16, RPL, 3, GM>, a, recb_smem_bytes<T>(a.N, GM), st, !GM);
+	return launch_dense(k_recb<T, 16, RPL, GM>, a, recb_smem_bytes<T>(a.N, GM), st, !GM);
 }
 
 template <typename T, bool GM>

@@ -820,146 +820,475 @@ struct RecArgs {
 	unsigned *err;
 };
 
-// The two triangular solves of the recombine for 8 real right-hand sides
-// c0 .. c0+7 (those < N) on the FP64 tensor cores, one warp: Y = D_b^-1 Q^H
-// with the LU's row order (perm), then L (unit lower) and U from M.  Rows go
-// by tiles of 8; the product of a tile's row of L (or U) with the tiles
-// already solved is a chain of m8n8k4 DMMAs (two accumulators), the 8 x 8
-// diagonal block is solved with shuffles.  Solved tiles are kept in the
-// B-fragment layout (lane: rows 4s + l%4, column l/4) for the later products.
-// ys: this warp's slab of 64 ceil(N/8) doubles in shared memory.  Tile t
-// of the solution is kept there in B layout (ys[64 t + 32 s + lane], k-step
-// s), each lane reading back only what it wrote, so the slab needs no
-// synchronisation; holding the tiles in registers instead spills.
-// osc: factors of the solution's rows on output (null: none).
-__device__ inline void recb_solve8(const double *M, int ld, const int *perm, const double *vsh,
-		const double *Q, double *G, int N, int c0, int lane, double *ys, const double *osc)
+// ----------------------------------------------- recombine
+//
+// G = (D_b^-1 Q^H + D_s T)^-1 D_b^-1 Q^H (greens.c:157-178), or its two-sided
+// form, one CTA per item with M in shared memory (GM: in global memory):
+//   * LU with partial pivoting in panels of 8 columns (getrf; the pivot is the
+//     first largest entry, in modulus for real and by |re| + |im| for complex
+//     scalars, as idamax / izamax).  The panel's warps hold it in registers,
+//     rows in place with their positions beside them.  A column costs one
+//     barrier among them: each warp leaves its candidate row in shared memory
+//     before it, and takes the winner's row from there after it.  They write
+//     the panel back in pivoted order and list the rows that moved.  The other
+//     warps meanwhile apply the previous panel to their tiles of 8 columns: the
+//     moved rows, the rows of U (substitution), the trailing rows by DMMA
+//     (one-panel look-ahead: the panel's warps bring its columns up to date in
+//     registers);
+//   * the 8 x 8 diagonal blocks of L and U are inverted in place, so that the
+//     solves have no divisions and no substitution;
+//   * each warp solves for 8 right-hand sides at a time, L and U by DMMA on
+//     tiles of 8 rows, solved tiles in a slab of shared memory (rec_solve8);
+//   * the phase 1/phase(det G) = phase(det Q) phase(det M) sign(prod v).
+// What bounds it: the panels' chain (N columns in turn), then the solve's
+// chains, of which the slabs that fit beside M limit how many run at once.
+// Two items, N = 144: 175 us a launch (LU 183k cycles, solves 130k), against 419 us
+// for an unblocked LU with a barrier per column and solves with substitution
+// in the diagonal blocks; 512 items 0.75 ms against 1.77; N = 256 (M in L2)
+// 1.09 ms against 6.0; complex N = 100 0.50 ms for 64 items against 1.12.
+
+// the magnitude a pivot is chosen by
+__device__ inline double pivot_mag(double a) { return fabs(a); }
+__device__ inline double pivot_mag(zd a) { return fabs(a.x) + fabs(a.y); }
+
+// the warps of a panel: one up to N = 64, else four; up to two rows a lane
+template <int RPL>
+struct LuPanel {
+	static constexpr int PW = RPL <= 2 ? 1 : 4;
+	static constexpr int RP = (RPL + PW - 1) / PW;
+};
+constexpr int LU_PB = 8;
+
+// the rows a panel moved: row src of the other columns goes to row dst
+struct LuMoves {
+	int n;
+	int src[16], dst[16];
+};
+
+// what a panel's warps share: the rows of U above it, their candidate rows
+// (two buffers)
+template <typename T>
+struct __align__(16) LuCand {
+	T u[LU_PB][LU_PB];              // rows of U in a panel's columns
+	T row[2][4][LU_PB];
+	unsigned long long key[2][4];
+	int pos[2][4];
+};
+
+// a panel's moved rows in the columns c0 .. c0+7 (those < cend), one warp
+template <typename T>
+__device__ inline void lu_move_tile(T *M, int ld, int c0, int cend, const LuMoves &mv, int lane)
 {
-	const int lr = lane & 3, lq = lane >> 2;
-	const int nt = (N + 7) / 8;
-	auto yb = [&](int u, int sgrp) -> double & { return ys[64 * u + 32 * sgrp + lane]; };
-	// C layout -> B layout of one tile: element (row r, col c) sits in lane
-	// 4 c + r % 4, k-step r / 4; lane (lq, lr) of the C layout holds rows lq,
-	// columns 2 lr + e
-	auto c_to_b = [&](double x0, double x1, double &b0, double &b1) {
+	const int c = c0 + (lane & 7), n = mv.n;
+	T v[4];
 #pragma unroll
-		for (int sgrp = 0; sgrp < 2; sgrp++) {
-			// B lane (lr', lq') wants row 4 sgrp + lr', column lq': in C it is
-			// lane 4 (4 sgrp + lr') + lq' / 2, element lq' % 2
-			const int src = 4 * (4 * sgrp + lr) + (lq >> 1);
-			const double v0 = __shfl_sync(0xffffffffu, x0, src), v1 = __shfl_sync(0xffffffffu, x1, src);
-			const double v = (lq & 1) ? v1 : v0;
-			if (sgrp == 0) b0 = v; else b1 = v;
-		}
-	};
-	auto b_to_c = [&](double b0, double b1, double &x0, double &x1) {
-		// C lane (lq, lr), element e: row lq, column 2 lr + e, held by B lane
-		// 4 (2 lr + e) + lq % 4 in k-step lq / 4
-#pragma unroll
-		for (int e = 0; e < 2; e++) {
-			const int src = 4 * (2 * lr + e) + (lq & 3);
-			const double v0 = __shfl_sync(0xffffffffu, b0, src), v1 = __shfl_sync(0xffffffffu, b1, src);
-			const double v = (lq < 4) ? v0 : v1;
-			if (e == 0) x0 = v; else x1 = v;
-		}
-	};
-	const int cc = c0 + 2 * lr;
-	// forward: L y = P Y
-#pragma unroll 1
-	for (int t = 0; t < nt; t++) {
-		const int r = 8 * t + lq;
-		double x[2];
-#pragma unroll
-		for (int e = 0; e < 2; e++) {
-			const int c = cc + e;
-			const int pr = (r < N) ? perm[r] : 0;
-			x[e] = (r < N && c < N) ? Q[c + (size_t)N * pr] * vsh[pr] : 0.0;
-		}
-		double a0[2] = {x[0], x[1]}, a1[2] = {0.0, 0.0};
-#pragma unroll 4
-		for (int u = 0; u < t; u++) {
-#pragma unroll
-			for (int sgrp = 0; sgrp < 2; sgrp++) {
-				const int k = 8 * u + 4 * sgrp + lr;
-				const double l = (r < N) ? -M[r + (size_t)ld * k] : 0.0;
-				if (sgrp == 0) dmma(a0[0], a0[1], l, yb(u, 0));
-				else dmma(a1[0], a1[1], l, yb(u, 1));
-			}
-		}
-		x[0] = a0[0] + a1[0];
-		x[1] = a0[1] + a1[1];
-		// unit lower 8 x 8 block
-#pragma unroll
-		for (int q = 0; q < 7; q++) {
-			const double y0 = __shfl_sync(0xffffffffu, x[0], 4 * q + lr);
-			const double y1 = __shfl_sync(0xffffffffu, x[1], 4 * q + lr);
-			if (lq > q && r < N) {
-				const double l = M[r + (size_t)ld * (8 * t + q)];
-				x[0] -= l * y0;
-				x[1] -= l * y1;
-			}
-		}
-		c_to_b(x[0], x[1], yb(t, 0), yb(t, 1));
+	for (int i = 0; i < 4; i++) {
+		const int m = (lane >> 3) + 4 * i;
+		if (m < n && c < cend) v[i] = M[mv.src[m] + (size_t)ld * c];
 	}
-	// backward: U g = y
-#pragma unroll 1
-	for (int t = nt - 1; t >= 0; t--) {
-		const int r = 8 * t + lq;
-		double x[2];
-		b_to_c(yb(t, 0), yb(t, 1), x[0], x[1]);
-		double a0[2] = {x[0], x[1]}, a1[2] = {0.0, 0.0};
-#pragma unroll 4
-		for (int u = t + 1; u < nt; u++) {
+	__syncwarp();
 #pragma unroll
-			for (int sgrp = 0; sgrp < 2; sgrp++) {
-				const int k = 8 * u + 4 * sgrp + lr;
-				const double uv = (r < N && k < N) ? -M[r + (size_t)ld * k] : 0.0;
-				if (sgrp == 0) dmma(a0[0], a0[1], uv, yb(u, 0));
-				else dmma(a1[0], a1[1], uv, yb(u, 1));
+	for (int i = 0; i < 4; i++) {
+		const int m = (lane >> 3) + 4 * i;
+		if (m < n && c < cend) M[mv.dst[m] + (size_t)ld * c] = v[i];
+	}
+	__syncwarp();
+}
+
+// named barrier 1 of the panel's warps
+template <int PW>
+__device__ inline void bar_lu()
+{
+	if (PW > 1) asm volatile("barrier.sync 1, %0;\n" ::"n"(PW * 32) : "memory");
+	else __syncwarp();
+}
+
+// LU of the panel of columns j0 .. j0+pb-1 (pb <= 8), rows j0 .. N-1, by the
+// warps w < PW: lane l of warp w holds the rows j0 + l + 32 (w + PW t).  With
+// mp (the moved rows of the panel before, 8 columns from j0 - 8) its columns
+// are brought up to date first, in the registers that then hold the panel.
+template <typename T, int RPL>
+__device__ inline void lu_panel(T *M, int ld, int N, int j0, int pb, int *ipiv, LuMoves &mv,
+		const LuMoves *mp, LuCand<T> &cd, int w, int lane, bool &nan_seen, bool &sing)
+{
+	constexpr int PW = LuPanel<RPL>::PW, RP = LuPanel<RPL>::RP, PB = LU_PB;
+	T x[RP][PB];
+	int pos[RP];
+	unsigned used = 0;
+	// the row slots that reach into the matrix (the same for the whole warp)
+	const int nslot = min(RP, (N - j0 - 32 * w + 32 * PW - 1) / (32 * PW));
+	if (w == 0 && lane == 0) mv.n = 0;
+	if (mp) {
+		if (w == 0) {
+			lu_move_tile(M, ld, j0, j0 + pb, *mp, lane);
+			// the rows of U: lane c column j0 + c
+			const int i0 = j0 - PB, c = lane & 7;
+			T u[PB];
+#pragma unroll
+			for (int i = 0; i < PB; i++) u[i] = c < pb ? M[i0 + i + (size_t)ld * (j0 + c)] : zero<T>();
+#pragma unroll
+			for (int k = 0; k < PB - 1; k++)
+#pragma unroll
+				for (int i = k + 1; i < PB; i++) u[i] -= M[i0 + i + (size_t)ld * (i0 + k)] * u[k];
+			if (lane < 8) {
+#pragma unroll
+				for (int i = 0; i < PB; i++) {
+					cd.u[i][c] = u[i];
+					if (c < pb) M[i0 + i + (size_t)ld * (j0 + c)] = u[i];
+				}
 			}
 		}
-		x[0] = a0[0] + a1[0];
-		x[1] = a0[1] + a1[1];
-		// upper 8 x 8 block, bottom up
+		bar_lu<PW>();
+	}
 #pragma unroll
-		for (int q = 7; q >= 0; q--) {
-			const int jq = 8 * t + q;
-			double ujj = (jq < N) ? M[jq + (size_t)ld * jq] : 1.0;
-			if (ujj == 0.0) ujj = 1.0;
-			if (lq == q) {
-				x[0] /= ujj;
-				x[1] /= ujj;
-			}
-			const double y0 = __shfl_sync(0xffffffffu, x[0], 4 * q + lr);
-			const double y1 = __shfl_sync(0xffffffffu, x[1], 4 * q + lr);
-			if (lq < q && r < N && jq < N) {
-				const double uv = M[r + (size_t)ld * jq];
-				x[0] -= uv * y0;
-				x[1] -= uv * y1;
+	for (int t = 0; t < RP; t++) {
+		const int r = j0 + lane + 32 * (w + PW * t);
+		pos[t] = r;
+		if (r >= N) used |= 1u << t;
+#pragma unroll
+		for (int c = 0; c < PB; c++) x[t][c] = (r < N && c < pb) ? M[r + (size_t)ld * (j0 + c)] : zero<T>();
+		if (mp && t < nslot) {
+			T l[PB];
+#pragma unroll
+			for (int k = 0; k < PB; k++) l[k] = r < N ? M[r + (size_t)ld * (j0 - PB + k)] : zero<T>();
+#pragma unroll
+			for (int k = 0; k < PB; k++)
+#pragma unroll
+				for (int c = 0; c < PB; c++) x[t][c] -= l[k] * cd.u[k][c];
+		}
+	}
+#pragma unroll
+	for (int k = 0; k < PB; k++) {
+		if (k >= pb) break;
+		// first largest of this warp's unused rows: by the bits of the magnitude
+		// (a NaN ranks last), then by position
+		unsigned long long best = 0;
+		int bp = 0x7fffffff, bt = 0;
+#pragma unroll
+		for (int t = 0; t < RP; t++) {
+			if (t >= nslot) break;
+			const double m = pivot_mag(x[t][k]);
+			const bool num = m >= 0.0, ok = !(used >> t & 1u);
+			if (ok && !num) nan_seen = true;
+			const unsigned long long key = num ? (unsigned long long)__double_as_longlong(m) : 0ull;
+			if (ok && (key > best || (key == best && pos[t] < bp))) {
+				best = key;
+				bp = pos[t];
+				bt = t;
 			}
 		}
+		const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
+		const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+		const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+		int q = __reduce_min_sync(0xffffffffu, (hi == mh && lo == ml) ? bp : 0x7fffffff);
+		if (bp == q) {
+			// its owner (every lane without rows when the warp has none left)
+#pragma unroll
+			for (int c = 0; c < PB; c++)
+				if (c >= k) cd.row[k & 1][w][c] = (RP > 1 && bt) ? x[RP - 1][c] : x[0][c];
+			cd.key[k & 1][w] = best;
+			cd.pos[k & 1][w] = bp;
+		}
+		bar_lu<PW>();
+		int ww = 0;
+		unsigned long long bk = cd.key[k & 1][0];
+		q = cd.pos[k & 1][0];
+#pragma unroll
+		for (int v = 1; v < PW; v++) {
+			const unsigned long long kv = cd.key[k & 1][v];
+			const int pv_ = cd.pos[k & 1][v];
+			if (kv > bk || (kv == bk && pv_ < q)) {
+				bk = kv;
+				q = pv_;
+				ww = v;
+			}
+		}
+		T pv[PB];
+#pragma unroll
+		for (int c = 0; c < PB; c++)
+			if (c >= k) pv[c] = cd.row[k & 1][ww][c];
+		T piv = pv[k];
+		if (re(piv) == 0.0 && im(piv) == 0.0) {
+			sing = true;
+			piv = one<T>();
+		}
+		const T ip = one<T>() / piv;
+		// positions: the pivot row to j, the row that was there to the pivot's
+		const int j = j0 + k;
+		if (w == 0 && lane == 0) ipiv[j] = q;
+#pragma unroll
+		for (int t = 0; t < RP; t++) {
+			if (t >= nslot) break;
+			const bool mine = pos[t] == q;
+			if (pos[t] == j) pos[t] = q;
+			if (mine) {
+				pos[t] = j;
+				used |= 1u << t;
+			}
+			if (!(used >> t & 1u)) {
+				x[t][k] = x[t][k] * ip;
+#pragma unroll
+				for (int c = 0; c < PB; c++)
+					if (c > k) x[t][c] -= x[t][k] * pv[c];
+			}
+		}
+	}
+#pragma unroll
+	for (int t = 0; t < RP; t++) {
+		if (t >= nslot) break;
+		const int r = j0 + lane + 32 * (w + PW * t);
 		if (r < N) {
-			const double f = osc ? osc[r] : 1.0;
-			if (cc < N) G[r + (size_t)N * cc] = x[0] * f;
-			if (cc + 1 < N) G[r + (size_t)N * (cc + 1)] = x[1] * f;
+#pragma unroll
+			for (int c = 0; c < PB; c++)
+				if (c < pb) M[pos[t] + (size_t)ld * (j0 + c)] = x[t][c];
 		}
-		c_to_b(x[0], x[1], yb(t, 0), yb(t, 1));
+		const bool moved = r < N && pos[t] != r;
+		const unsigned m = __ballot_sync(0xffffffffu, moved);
+		int i = 0;
+		if (m && lane == 0) i = atomicAdd(&mv.n, __popc(m));
+		i = __shfl_sync(0xffffffffu, i, 0) + __popc(m & ((1u << lane) - 1u));
+		if (moved) {
+			mv.src[i] = r;
+			mv.dst[i] = pos[t];
+		}
 	}
 }
 
-// ----------------------------------------------- recombine in shared memory
-//
-// G = (D_b^-1 Q^H + D_s T)^-1 D_b^-1 Q^H (greens.c:157-178)
-// with M in shared memory: LU with partial pivoting and physical row swaps
-// (getrf: the first largest |M[r, j]| of the column, as idamax); warp 0
-// picks, swaps and scales, all warps update the trailing columns.  Then
-// each warp solves for its right-hand sides, CB at a time held in
-// registers (permutation, unit-lower forward, upper backward), and the
-// phase 1/phase(det G) = phase(det Q) phase(det M) sign(prod v).
+// C layout -> B layout of an 8 x 8 tile: element (row r, col c) sits in lane
+// 4 c + r % 4, k-step r / 4; lane (lq, lr) of the C layout holds row lq, columns
+// 2 lr + e
+template <typename T>
+__device__ inline void tile_c_to_b(const T (&x)[2], T (&b)[2], int lane)
+{
+	const int lr = lane & 3, lq = lane >> 2;
+#pragma unroll
+	for (int s = 0; s < 2; s++) {
+		const int src = 4 * (4 * s + lr) + (lq >> 1);
+		const T v0 = shfl(x[0], src), v1 = shfl(x[1], src);
+		b[s] = (lq & 1) ? v1 : v0;
+	}
+}
 
-// the recombine's shared memory: M (unless in global memory), the scale
-// vectors and pivots, then (real M in shared memory) the solve slabs of
-// recb_solve_warps warps, as many as fit under RECB_SMEM_CAP, at least one
+template <typename T>
+__device__ inline void tile_b_to_c(const T (&b)[2], T (&x)[2], int lane)
+{
+	// C lane (lq, lr), element e: row lq, column 2 lr + e, held by B lane
+	// 4 (2 lr + e) + lq % 4 in k-step lq / 4
+	const int lr = lane & 3, lq = lane >> 2;
+#pragma unroll
+	for (int e = 0; e < 2; e++) {
+		const int src = 4 * (2 * lr + e) + (lq & 3);
+		const T v0 = shfl(b[0], src), v1 = shfl(b[1], src);
+		x[e] = (lq < 4) ? v0 : v1;
+	}
+}
+
+// c (8 x 8 accumulators) += a b, one k-step
+__device__ inline void tile_mma(double (&c)[2], double a, double b) { dmma(c[0], c[1], a, b); }
+__device__ inline void tile_mma(zd (&c)[2], zd a, zd b)
+{
+	dmma(c[0].x, c[1].x, a.x, b.x);
+	dmma(c[0].x, c[1].x, -a.y, b.y);
+	dmma(c[0].y, c[1].y, a.x, b.y);
+	dmma(c[0].y, c[1].y, a.y, b.x);
+}
+
+// the rows j0 .. j0+pb-1 of U in the columns c0 .. c0+7 (those < N) right of
+// the panel, from the moved rows by substitution, one warp; returns them as a
+// B operand
+template <typename T>
+__device__ inline void lu_u_rows(T *M, int ld, int N, int j0, int pb, int c0, int lane, T (&b)[2])
+{
+	constexpr int PB = LU_PB;
+	const int lr = lane & 3, lq = lane >> 2, cc = c0 + 2 * lr;
+	const bool in = lq < pb;
+	T l[PB - 1], u[2];
+#pragma unroll
+	for (int q = 0; q < PB - 1; q++) l[q] = (in && q < lq) ? M[j0 + lq + (size_t)ld * (j0 + q)] : zero<T>();
+#pragma unroll
+	for (int e = 0; e < 2; e++) u[e] = (in && cc + e < N) ? M[j0 + lq + (size_t)ld * (cc + e)] : zero<T>();
+#pragma unroll
+	for (int q = 0; q < PB - 1; q++) {
+		const T y0 = shfl(u[0], 4 * q + lr), y1 = shfl(u[1], 4 * q + lr);
+		u[0] -= l[q] * y0;
+		u[1] -= l[q] * y1;
+	}
+#pragma unroll
+	for (int e = 0; e < 2; e++)
+		if (in && cc + e < N) M[j0 + lq + (size_t)ld * (cc + e)] = u[e];
+	tile_c_to_b(u, b, lane);
+}
+
+// M -= L U on the rows from j0 + pb on of the columns c0 .. c0+7, one warp
+template <typename T>
+__device__ inline void lu_trail(T *M, int ld, int N, int j0, int pb, int c0, const T (&b)[2], int lane)
+{
+	constexpr int RT = is_cplx<T>::value ? 2 : 3;   // row tiles at a time
+	const int lr = lane & 3, lq = lane >> 2, cc = c0 + 2 * lr;
+	for (int r0 = j0 + pb; r0 < N; r0 += 8 * RT) {
+		T x[RT][2], a[RT][2];
+		T *Mx = M + r0 + lq + (size_t)ld * cc;
+		const T *Ma = M + r0 + lq + (size_t)ld * (j0 + lr);
+#pragma unroll
+		for (int i = 0; i < RT; i++) {
+			const bool in = r0 + 8 * i + lq < N;
+#pragma unroll
+			for (int e = 0; e < 2; e++) x[i][e] = (in && cc + e < N) ? Mx[8 * i + ld * e] : zero<T>();
+#pragma unroll
+			for (int s = 0; s < 2; s++) a[i][s] = (in && 4 * s + lr < pb) ? -Ma[8 * i + ld * 4 * s] : zero<T>();
+		}
+#pragma unroll
+		for (int s = 0; s < 2; s++)
+#pragma unroll
+			for (int i = 0; i < RT; i++) tile_mma(x[i], a[i][s], b[s]);
+#pragma unroll
+		for (int i = 0; i < RT; i++) {
+			const bool in = r0 + 8 * i + lq < N;
+#pragma unroll
+			for (int e = 0; e < 2; e++)
+				if (in && cc + e < N) Mx[8 * i + ld * e] = x[i][e];
+		}
+	}
+	__syncwarp();
+}
+
+// inverse in place of an 8 x 8 diagonal block: of unit lower L (below the
+// diagonal) or of U (on and above it), one warp, lane c < 8 column c
+template <typename T, bool LOWER>
+__device__ inline void tri_invert8(T *M, int ld, int N, int j0, int lane)
+{
+	const int c = lane & 7;
+	T x[8];
+	if (LOWER) {
+#pragma unroll
+		for (int i = 0; i < 8; i++) {
+			T v = (i == c) ? one<T>() : zero<T>();
+#pragma unroll
+			for (int k = 0; k < i; k++) {
+				const T l = (j0 + i < N) ? M[j0 + i + (size_t)ld * (j0 + k)] : zero<T>();
+				v -= l * x[k];
+			}
+			x[i] = v;
+		}
+	} else {
+		T d = (j0 + c < N) ? M[j0 + c + (size_t)ld * (j0 + c)] : one<T>();
+		if (re(d) == 0.0 && im(d) == 0.0) d = one<T>();
+		d = one<T>() / d;
+#pragma unroll
+		for (int i = 7; i >= 0; i--) {
+			T v = (i == c) ? one<T>() : zero<T>();
+#pragma unroll
+			for (int k = 7; k > i; k--) {
+				const T u = (j0 + k < N) ? M[j0 + i + (size_t)ld * (j0 + k)] : zero<T>();
+				v -= u * x[k];
+			}
+			x[i] = v * shfl(d, i);
+		}
+	}
+	__syncwarp();
+#pragma unroll
+	for (int i = 0; i < 8; i++)
+		if (lane < 8 && j0 + i < N && j0 + c < N && (LOWER ? i > c : i <= c)) M[j0 + i + (size_t)ld * (j0 + c)] = x[i];
+}
+
+// The two triangular solves for the right-hand sides c0 .. c0+7 (those < N),
+// one warp: Y = D_b^-1 Q^H with the LU's row order (perm), then L and U from M,
+// whose 8 x 8 diagonal blocks are inverted.  Rows go by tiles of 8: the
+// product of a tile's row of L (or U) with the tiles already solved is a chain
+// of DMMAs (two accumulators), the diagonal block one product more.  Solved
+// tiles are kept in the B-fragment layout (lane: rows 4s + l%4, column l/4)
+// in ys, this warp's slab of 64 ceil(N/8) numbers in shared memory, each lane
+// reading back only what it wrote.  osc: factors of the solution's rows on
+// output (null: none).  UN: tiles whose loads are on their way together.
+template <typename T, int UN>
+__device__ inline void rec_solve8(const T *M, int ld, const int *perm, const double *vsh, const T *Q,
+		T *G, int N, int c0, int lane, T *ys, const double *osc)
+{
+	const int lr = lane & 3, lq = lane >> 2, cc = c0 + 2 * lr;
+	const int nt = (N + 7) / 8;
+	auto yb = [&](int u, int s) -> T & { return ys[64 * u + 32 * s + lane]; };
+	// rows past N take row N - 1's entries of M: their results stay finite and
+	// are not used (their columns of L and U count as zero)
+	T xn[2];
+	double vn;
+	auto rhs = [&](int t) {
+		const int pr = perm[min(8 * t + lq, N - 1)];
+		vn = vsh[pr];
+#pragma unroll
+		for (int e = 0; e < 2; e++) xn[e] = Q[min(cc + e, N - 1) + (size_t)N * pr];
+	};
+	rhs(0);
+#pragma unroll 1
+	for (int t = 0; t < nt; t++) {
+		const T *Mr = M + min(8 * t + lq, N - 1) + (size_t)ld * lr;
+		const T x0 = conjv(xn[0]) * vn, x1 = conjv(xn[1]) * vn;
+		T a0[2] = {zero<T>(), zero<T>()}, a1[2] = {zero<T>(), zero<T>()}, b[2];
+		T y[2] = {zero<T>(), zero<T>()};
+		if (t + 1 < nt) rhs(t + 1);
+		// the diagonal block's inverse, on its way meanwhile
+		const T *Md = Mr + (size_t)ld * 8 * t;
+		const bool in = 8 * t + lq < N;
+		T ld0 = (in && lr < lq) ? Md[0] : zero<T>(), ld1 = (in && lr + 4 < lq) ? Md[(size_t)ld * 4] : zero<T>();
+		if (lr == lq) ld0 = one<T>();
+		if (lr + 4 == lq) ld1 = one<T>();
+#pragma unroll UN
+		for (int u = 0; u < t; u++) {
+			const T l0 = Mr[0], l1 = Mr[(size_t)ld * 4];
+			Mr += (size_t)ld * 8;
+			tile_mma(a0, l0, yb(u, 0));
+			tile_mma(a1, l1, yb(u, 1));
+		}
+		a0[0] = x0 - (a0[0] + a1[0]);
+		a0[1] = x1 - (a0[1] + a1[1]);
+		tile_c_to_b(a0, b, lane);
+		tile_mma(y, ld0, b[0]);
+		tile_mma(y, ld1, b[1]);
+		tile_c_to_b(y, b, lane);
+		yb(t, 0) = b[0];
+		yb(t, 1) = b[1];
+	}
+#pragma unroll 1
+	for (int t = nt - 1; t >= 0; t--) {
+		const int r = 8 * t + lq;
+		const T *Md = M + min(r, N - 1) + (size_t)ld * (8 * t + lr), *Mr = Md + (size_t)ld * 8;
+		T a0[2] = {zero<T>(), zero<T>()}, a1[2] = {zero<T>(), zero<T>()}, b[2] = {yb(t, 0), yb(t, 1)};
+		T y[2] = {zero<T>(), zero<T>()}, x[2];
+		const T ud0 = (lr >= lq && 8 * t + lr < N) ? Md[0] : zero<T>();
+		const T ud1 = (lr + 4 >= lq && 8 * t + lr + 4 < N) ? Md[(size_t)ld * 4] : zero<T>();
+		tile_b_to_c(b, x, lane);
+		// columns past N: only in the last tile
+#pragma unroll UN
+		for (int u = t + 1; u < nt - 1; u++) {
+			const T u0 = Mr[0], u1 = Mr[(size_t)ld * 4];
+			Mr += (size_t)ld * 8;
+			tile_mma(a0, u0, yb(u, 0));
+			tile_mma(a1, u1, yb(u, 1));
+		}
+		if (t + 1 < nt) {
+			const int k = 8 * (nt - 1) + lr;
+			const T u0 = k < N ? Mr[0] : zero<T>(), u1 = k + 4 < N ? Mr[(size_t)ld * 4] : zero<T>();
+			tile_mma(a0, u0, yb(nt - 1, 0));
+			tile_mma(a1, u1, yb(nt - 1, 1));
+		}
+		a0[0] = x[0] - (a0[0] + a1[0]);
+		a0[1] = x[1] - (a0[1] + a1[1]);
+		tile_c_to_b(a0, b, lane);
+		tile_mma(y, ud0, b[0]);
+		tile_mma(y, ud1, b[1]);
+		if (r < N) {
+			const double f = osc ? osc[r] : 1.0;
+			if (cc < N) G[r + (size_t)N * cc] = y[0] * f;
+			if (cc + 1 < N) G[r + (size_t)N * (cc + 1)] = y[1] * f;
+		}
+		tile_c_to_b(y, b, lane);
+		yb(t, 0) = b[0];
+		yb(t, 1) = b[1];
+	}
+}
+
+// shared memory: M (unless in global memory), the scale vectors, pivots, row
+// order and move lists, then the solve slabs of rec_solve_warps warps, as many
+// as fit under RECB_SMEM_CAP, at least one
 constexpr size_t RECB_SMEM_CAP = 226 * 1024;
 
 template <typename T>
@@ -967,16 +1296,16 @@ __host__ __device__ inline size_t recb_base_bytes(int N, bool gm)
 {
 	// a multiple of 16 bytes, where the solve slabs start
 	return ((gm ? 0 : sizeof(T) * (size_t)qrb_ld(N) * N) + sizeof(double) * 2 * (size_t)N
-	        + sizeof(int) * 2 * (size_t)N + 64 + 15) & ~(size_t)15;
+	        + sizeof(int) * 2 * (size_t)N + 2 * sizeof(LuMoves) + sizeof(LuCand<T>) + 64 + 31) & ~(size_t)15;
 }
 
-__host__ __device__ inline size_t recb_slab_bytes(int N) { return sizeof(double) * 64 * (size_t)((N + 7) / 8); }
+template <typename T>
+__host__ __device__ inline size_t recb_slab_bytes(int N) { return sizeof(T) * 64 * (size_t)((N + 7) / 8); }
 
 template <typename T>
 __host__ __device__ inline int recb_solve_warps(int N, bool gm)
 {
-	if (is_cplx<T>::value || gm) return 0;
-	const size_t base = recb_base_bytes<T>(N, gm), slab = recb_slab_bytes(N);
+	const size_t base = recb_base_bytes<T>(N, gm), slab = recb_slab_bytes<T>(N);
 	const size_t fit = base < RECB_SMEM_CAP ? (RECB_SMEM_CAP - base) / slab : 0;
 	return fit < 1 ? 1 : (fit > 16 ? 16 : (int)fit);
 }
@@ -984,12 +1313,13 @@ __host__ __device__ inline int recb_solve_warps(int N, bool gm)
 template <typename T>
 size_t recb_smem_bytes(int N, bool gm = false)
 {
-	return recb_base_bytes<T>(N, gm) + recb_slab_bytes(N) * recb_solve_warps<T>(N, gm);
+	return recb_base_bytes<T>(N, gm) + recb_slab_bytes<T>(N) * recb_solve_warps<T>(N, gm);
 }
 
-template <typename T, int NW, int RPL, int CB, bool GM>
+template <typename T, int NW, int RPL, bool GM>
 __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 {
+	constexpr int PB = LU_PB, PW = LuPanel<RPL>::PW;
 	const int item = blockIdx.x;
 	if (item >= a.batch) return;
 	const int N = a.N, ld = GM ? N : qrb_ld(N);
@@ -997,10 +1327,12 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 	extern __shared__ __align__(16) unsigned char smraw[];
 	// N columns, leading dimension ld
 	T *M = GM ? a.work + (size_t)item * a.w_stride : (T *)smraw;
-	double *vsh = GM ? (double *)smraw : (double *)(M + (size_t)ld * N);   // D_b^-1
-	double *dss = vsh + N;                      // D_s
+	double *vsh = GM ? (double *)smraw : (double *)((T *)smraw + (size_t)ld * N);   // D_b^-1
+	double *dss = vsh + N;                      // D_s, then (two-sided) D_Lb^-1
 	int *ipiv = (int *)(dss + N);               // row swapped with row j at step j
 	int *perm = ipiv + N;                       // row r of P Y is row perm[r] of Y
+	LuMoves *mv = (LuMoves *)(perm + N);        // of panel p, by parity
+	LuCand<T> &cd = *(LuCand<T> *)(((size_t)(mv + 2) + 15) & ~(size_t)15);
 	if (N > 32 * RPL) {
 		if (tid == 0 && a.err) atomicOr(a.err, DQ_ERR_SIZE);
 		return;
@@ -1012,6 +1344,7 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 		const double dr = d[r];
 		if (fabs(dr) > 1.0) { vsh[r] = 1.0 / dr; dss[r] = 1.0; }
 		else { vsh[r] = 1.0; dss[r] = dr; }
+		perm[r] = r;
 	}
 	__syncthreads();
 	const double *osc = nullptr;
@@ -1036,190 +1369,43 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 	__syncthreads();
 
 	bool nan_seen = false, sing = false;
-	// Pivot of column j (warp 0): the first largest |M[r, j]|, r >= j, as
-	// idamax; rows j and the pivot row swapped in column j only (the other
-	// columns swap them when step j reaches them); multipliers scaled.
-	auto pivot_col = [&](int j) {
-		double best = -1.0;
-		int br = N;
-		for (int r = j + lane; r < N; r += 32) {
-			double m = absv(M[r + (size_t)ld * j]);
-			if (!(m >= 0.0)) {
-				m = -0.5;
-				nan_seen = true;
-			}
-			if (m > best) { best = m; br = r; }
-		}
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) {
-			const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-			const int orr = __shfl_xor_sync(0xffffffffu, br, o);
-			if (ob > best || (ob == best && orr < br)) { best = ob; br = orr; }
-		}
-		if (lane == 0) {
-			if (br != j) {
-				const T t0 = M[j + (size_t)ld * j];
-				M[j + (size_t)ld * j] = M[br + (size_t)ld * j];
-				M[br + (size_t)ld * j] = t0;
-			}
-			ipiv[j] = br;
-		}
-		__syncwarp();
-		T piv = M[j + (size_t)ld * j];
-		if (re(piv) == 0.0 && im(piv) == 0.0) {
-			sing = true;
-			piv = one<T>();
-		}
-		const T ip = one<T>() / piv;
-		for (int r = j + 1 + lane; r < N; r += 32) M[r + (size_t)ld * j] *= ip;
-	};
-	// Step j on column c > j (one warp): the row swap of step j, then the
-	// rank-1 update with the multipliers l of column j
-	auto update_col = [&](int j, int pj, int c, const T (&l)[RPL]) {
-		T *col = M + (size_t)ld * c;
-		if (lane == 0 && pj != j) {
-			const T t0 = col[j];
-			col[j] = col[pj];
-			col[pj] = t0;
-		}
-		__syncwarp();
-		const T u = col[j];
-#pragma unroll
-		for (int t = 0; t < RPL; t++) {
-			const int r = j + 1 + lane + 32 * t;
-			if (r < N) col[r] -= l[t] * u;
-		}
-	};
-	// One barrier per step: warp 0 updates column j + 1 and pivots it for
-	// the next step (look-ahead) while warps 1.. update the other columns and
-	// apply the step's row swap to the columns left of j (the L factor).
-	if (w == 0) pivot_col(0);
+	if (w < PW) lu_panel<T, RPL>(M, ld, N, 0, min(PB, N), ipiv, mv[0], nullptr, cd, w, lane, nan_seen, sing);
 	__syncthreads();
-	for (int j = 0; j < N; j++) {
-		const int pj = ipiv[j];
-		T l[RPL];
-#pragma unroll
-		for (int t = 0; t < RPL; t++) {
-			const int r = j + 1 + lane + 32 * t;
-			l[t] = (r < N) ? M[r + (size_t)ld * j] : zero<T>();
-		}
-		if (w == 0) {
-			if (j + 1 < N) {
-				update_col(j, pj, j + 1, l);
-				__syncwarp();
-				pivot_col(j + 1);
-			}
+	for (int j0 = 0, p = 0; j0 < N; j0 += PB, p++) {
+		const int pb = min(PB, N - j0), j1 = j0 + pb;
+		const LuMoves &m = mv[p & 1];
+		if (w < PW) {
+			if (j1 < N)
+				lu_panel<T, RPL>(M, ld, N, j1, min(PB, N - j1), ipiv, mv[(p + 1) & 1], &m, cd, w, lane, nan_seen,
+				                 sing);
 		} else {
-			if (pj != j)
-				for (int c = tid - 32; c < j; c += blockDim.x - 32) {
-					const T t0 = M[j + (size_t)ld * c];
-					M[j + (size_t)ld * c] = M[pj + (size_t)ld * c];
-					M[pj + (size_t)ld * c] = t0;
+			if (w == NW - 1) {
+				const int v = lane < m.n ? perm[m.src[lane & 15]] : 0;
+				__syncwarp();
+				if (lane < m.n) perm[m.dst[lane]] = v;
+			}
+			// tiles right of the next panel, then the columns left of this one
+			const int nr = max(0, (N - (j1 + 8) + 7) / 8), nl = m.n ? (j0 + 7) / 8 : 0;
+			for (int t = w - PW; t < nr + nl; t += NW - PW) {
+				if (t < nr) {
+					const int c0 = j1 + 8 + 8 * t;
+					T b[2];
+					lu_move_tile(M, ld, c0, N, m, lane);
+					lu_u_rows<T>(M, ld, N, j0, pb, c0, lane, b);
+					lu_trail<T>(M, ld, N, j0, pb, c0, b, lane);
+				} else {
+					lu_move_tile(M, ld, 8 * (t - nr), j0, m, lane);
 				}
-			for (int c = j + 1 + w; c < N; c += NW - 1) update_col(j, pj, c, l);
+			}
 		}
 		__syncthreads();
 	}
-	nan_seen = __any_sync(0xffffffffu, nan_seen);
-	sing = __any_sync(0xffffffffu, sing);
-	if (tid == 0) {
-		for (int r = 0; r < N; r++) perm[r] = r;
-		for (int j = 0; j < N; j++) {
-			const int q = ipiv[j];
-			const int t0 = perm[j];
-			perm[j] = perm[q];
-			perm[q] = t0;
-		}
-	}
-	if (w == 0 && lane == 0) {
-		if (nan_seen && a.err) atomicOr(a.err, DQ_ERR_NAN);
-		if (sing && a.err) atomicOr(a.err, DQ_ERR_SINGULAR);
-	}
-	__syncthreads();
-
-	// right-hand sides Y = D_b^-1 Q^H, CB columns per pass of a warp
-	T *G = a.G + (size_t)item * a.g_stride;
-	constexpr bool TC = !is_cplx<T>::value && !GM;   // real, shared memory: DMMA tiles
-	if constexpr (TC) {
-		const int nws = min(NW, recb_solve_warps<T>(N, GM));
-		double *ys = (double *)(smraw + recb_base_bytes<T>(N, GM))
-		             + (size_t)64 * ((N + 7) / 8) * w;
-		for (int c0 = 8 * w; w < nws && c0 < N; c0 += 8 * nws)
-			recb_solve8((const double *)M, ld, perm, vsh, (const double *)Q, (double *)G, N, c0,
-			                     lane, ys, osc);
-	}
-	for (int c0 = w * CB; !TC && c0 < N; c0 += NW * CB) {
-		T y[CB][RPL];
-#pragma unroll
-		for (int b = 0; b < CB; b++) {
-			const int c = c0 + b;
-#pragma unroll
-			for (int t = 0; t < RPL; t++) {
-				const int r = lane + 32 * t;
-				const int pr = (r < N) ? perm[r] : 0;
-				y[b][t] = (c < N && r < N) ? conjv(Q[c + (size_t)N * pr]) * vsh[pr] : zero<T>();
-			}
-		}
-		// L (unit lower)
-		for (int k = 0; k < N - 1; k++) {
-			const int tk = k >> 5, lk = k & 31;
-			T yk[CB];
-#pragma unroll
-			for (int b = 0; b < CB; b++) {
-				T v = zero<T>();
-#pragma unroll
-				for (int t = 0; t < RPL; t++)
-					if (t == tk) v = y[b][t];
-				yk[b] = shfl(v, lk);
-			}
-#pragma unroll
-			for (int t = 0; t < RPL; t++) {
-				const int r = lane + 32 * t;
-				if (r > k && r < N) {
-					const T lv = M[r + (size_t)ld * k];
-#pragma unroll
-					for (int b = 0; b < CB; b++) y[b][t] -= lv * yk[b];
-				}
-			}
-		}
-		// U
-		for (int k = N - 1; k >= 0; k--) {
-			const int tk = k >> 5, lk = k & 31;
-			T ukk = M[k + (size_t)ld * k];
-			if (re(ukk) == 0.0 && im(ukk) == 0.0) ukk = one<T>();
-			const T iu = one<T>() / ukk;
-			T yk[CB];
-#pragma unroll
-			for (int b = 0; b < CB; b++) {
-				T v = zero<T>();
-#pragma unroll
-				for (int t = 0; t < RPL; t++)
-					if (t == tk) v = y[b][t];
-				yk[b] = shfl(v, lk) * iu;
-			}
-#pragma unroll
-			for (int t = 0; t < RPL; t++) {
-				const int r = lane + 32 * t;
-				if (r < k) {
-					const T uv = M[r + (size_t)ld * k];
-#pragma unroll
-					for (int b = 0; b < CB; b++) y[b][t] -= uv * yk[b];
-				} else if (r == k) {
-#pragma unroll
-					for (int b = 0; b < CB; b++) y[b][t] = yk[b];
-				}
-			}
-		}
-#pragma unroll
-		for (int b = 0; b < CB; b++) {
-			const int c = c0 + b;
-			if (c >= N) continue;
-#pragma unroll
-			for (int t = 0; t < RPL; t++) {
-				const int r = lane + 32 * t;
-				if (r < N) G[r + (size_t)N * c] = osc ? y[b][t] * osc[r] : y[b][t];
-			}
-		}
+	// any panel warp may have met a NaN or a zero pivot
+	if (w < PW) {
+		nan_seen = __any_sync(0xffffffffu, nan_seen);
+		sing = __any_sync(0xffffffffu, sing);
+		if (lane == 0 && nan_seen && a.err) atomicOr(a.err, DQ_ERR_NAN);
+		if (w == 0 && lane == 0 && sing && a.err) atomicOr(a.err, DQ_ERR_SINGULAR);
 	}
 	if (w == 0) {
 		// phase(det) = phase(det Q) prod phase(U_jj) sign(prod v_j) (-1)^swaps,
@@ -1248,6 +1434,19 @@ __global__ void __launch_bounds__(NW * 32) k_recb(RecArgs<T> a)
 			if (a.logdet) a.logdet[item] = l;
 		}
 	}
+	__syncthreads();
+	const int nt = (N + 7) / 8;
+	for (int t = w; t < 2 * nt; t += NW) {
+		if (t < nt) tri_invert8<T, true>(M, ld, N, 8 * t, lane);
+		else tri_invert8<T, false>(M, ld, N, 8 * (t - nt), lane);
+	}
+	__syncthreads();
+	// right-hand sides Y = D_b^-1 Q^H, 8 columns per pass of a warp
+	T *G = a.G + (size_t)item * a.g_stride;
+	const int nws = min(NW, recb_solve_warps<T>(N, GM));
+	T *ys = (T *)(smraw + recb_base_bytes<T>(N, GM)) + (size_t)64 * nt * w;
+	for (int c0 = 8 * w; w < nws && c0 < N; c0 += 8 * nws)
+		rec_solve8<T, GM ? 8 : 4>(M, ld, perm, vsh, Q, G, N, c0, lane, ys, osc);
 }
 
 }  // namespace dq

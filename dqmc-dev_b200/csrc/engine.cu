@@ -1262,8 +1262,12 @@ struct Group : GroupBase, ProfHook {
 	// further off than the whole chain's (12x12, beta = 6: 5e-14 against
 	// 1.3e-13; 8x8, U = 6, beta = 8 from random fields: 7e-11 against 1e-8).
 
-	// one factorisation: X (or X^H) -> Q, diag, T; prev: the columns' scales
-	// and T so far (null: the first factor, column-pivoted)
+	// one factorisation: X (or X^H) -> Q, diag, T, the columns taken in order
+	// of their norms; prev: the columns' scales and T so far (null: the first
+	// factor).  greens.c:89 pivots the first factor column by column; taking
+	// its order from the initial norms as all later ones leaves the error of G
+	// as it was and the launch of k_qrb in place of k_qrp (us, two items:
+	// N = 144 270 for 680, N = 256 1480 for 4440)
 	int qdt(const T *Xin, long long xs, bool trans, const double *dprev, const T *Tprev, T *Q, double *d,
 	        T *Tout, T *qd)
 	{
@@ -1278,7 +1282,7 @@ struct Group : GroupBase, ProfHook {
 		q.qdet = qd;
 		q.pvt = pvt.p; q.p_stride = N;
 		q.work = W.p; q.w_stride = NN;
-		q.mode = dprev ? QR_PRESORT : QR_PIVOT;
+		q.mode = QR_PRESORT;
 		if (dprev) {
 			q.dcol = dprev; q.d_stride = N;
 			q.Rs = Rs.p; q.r_stride = NN;
@@ -1287,7 +1291,7 @@ struct Group : GroupBase, ProfHook {
 		}
 		prof_begin(0);
 		if (launch_qr<T>(q, st)) return DQMC_E_ARG;
-		prof_end(dprev ? PC_QR_PRESORT : PC_QR_PIVOT, qfl, qby);
+		prof_end(PC_QR_PRESORT, qfl, qby);
 		launch_count++;
 		if (!dprev) return 0;
 		GemmArgs<T> g = gargs<T>(N, N, N, NB, Rs.p, per_item(NN), N, Tprev, per_item(NN), N, Tout, per_item(NN),

@@ -27,10 +27,10 @@ template <typename T>
 struct QrArgs {
 	int N, batch, mode;
 	const T *X; long long x_stride;       // input matrices (ld N)
-	int trans;                            // PIVOT: factor X^H instead of X
-	const double *dcol; long long d_stride; // PRESORT: columns scaled by d on load
+	int trans;                            // PRESORT: factor X^H instead of X
+	const double *dcol; long long d_stride; // PRESORT: columns scaled by d on load (null: 1)
 	T *Q; long long q_stride;             // explicit Q out
-	T *Tout; long long t_stride;          // PIVOT: T = D^-1 R P^T
+	T *Tout; long long t_stride;          // T = D^-1 R P^T (PRESORT: or Rs)
 	T *Rs; long long r_stride;            // PRESORT: D^-1 R in pivot order
 	int *pvt; long long p_stride;         // pivot order (column chosen at step j)
 	double *dout; long long dout_stride;  // diag(R), 0 -> 1 (real: Householder beta)
@@ -317,14 +317,34 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 		return;
 	}
 	const T *X = a.X + (size_t)item * a.x_stride;
-	const double *dc = a.dcol + (size_t)item * a.d_stride;
+	const double *dc = a.dcol ? a.dcol + (size_t)item * a.d_stride : nullptr;
 
-	for (int c = w; c < N; c += NW) {
-		const double sc = dc[c];
-		double s = 0.0;
-		for (int r = lane; r < N; r += 32) s += abs2(X[r + (size_t)N * c] * sc);
-		s = warp_sum(s);
-		if (lane == 0) vn[c] = s;
+	if (a.trans) {
+		// norms of X's rows: a warp's lanes take 32 rows, a warp every NW-th column,
+		// the partial sums meet in Vb
+		const int nrow = (N + 31) / 32, g = w / nrow, ng = min(NW / nrow, NBK);
+		double *ps = (double *)Vb;
+		const int c = (w - g * nrow) * 32 + lane;
+		if (g < ng && c < N) {
+			double s = 0.0;
+#pragma unroll 4
+			for (int r = g; r < N; r += ng) s += abs2(X[c + (size_t)N * r]);
+			ps[g * N + c] = s;
+		}
+		__syncthreads();
+		for (int q = tid; q < N; q += blockDim.x) {
+			double s = 0.0;
+			for (int k = 0; k < ng; k++) s += ps[k * N + q];
+			vn[q] = dc ? s * dc[q] * dc[q] : s;
+		}
+	} else {
+		for (int c = w; c < N; c += NW) {
+			const double sc = dc ? dc[c] : 1.0;
+			double s = 0.0;
+			for (int r = lane; r < N; r += 32) s += abs2(X[r + (size_t)N * c] * sc);
+			s = warp_sum(s);
+			if (lane == 0) vn[c] = s;
+		}
 	}
 	__syncthreads();
 	// stable descending order of the squared norms (greens.c:123-129); a NaN
@@ -342,12 +362,20 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 			rank += (u > v) || (u == v && o < c);
 		}
 		pvt[rank] = c;
+		if (a.trans) ((int *)Vb)[c] = rank;
 	}
 	__syncthreads();
-	for (int j = w; j < N; j += NW) {
-		const int c = pvt[j];
-		const double sc = dc[c];
-		for (int r = lane; r < N; r += 32) A[r + (size_t)ld * j] = X[r + (size_t)N * c] * sc;
+	if (a.trans) {
+		const int *rk = (const int *)Vb;
+		for (int r = w; r < N; r += NW)
+			for (int c = lane; c < N; c += 32)
+				A[r + (size_t)ld * rk[c]] = conjv(X[c + (size_t)N * r]) * (dc ? dc[c] : 1.0);
+	} else {
+		for (int j = w; j < N; j += NW) {
+			const int c = pvt[j];
+			const double sc = dc ? dc[c] : 1.0;
+			for (int r = lane; r < N; r += 32) A[r + (size_t)ld * j] = X[r + (size_t)N * c] * sc;
+		}
 	}
 	__syncthreads();
 
@@ -478,13 +506,16 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 		__syncthreads();
 	}
 
-	// D^-1 R in position order, diag(R) (0 -> 1) and the order
-	for (int j = w; j < N; j += NW)
+	// D^-1 R in position order (Rs) or in the original one (Tout), diag(R)
+	// (0 -> 1) and the order
+	for (int j = w; j < N; j += NW) {
+		T *out = a.Tout ? a.Tout + (size_t)item * a.t_stride + (size_t)N * pvt[j]
+		                : a.Rs + (size_t)item * a.r_stride + (size_t)N * j;
 		for (int r = lane; r < N; r += 32) {
 			const double dr = dsh[r] == 0.0 ? 1.0 : dsh[r];
-			a.Rs[(size_t)item * a.r_stride + r + (size_t)N * j] =
-				(r <= j) ? A[r + (size_t)ld * j] / dr : zero<T>();
+			out[r] = (r <= j) ? A[r + (size_t)ld * j] / dr : zero<T>();
 		}
+	}
 	for (int r = tid; r < N; r += blockDim.x) {
 		a.dout[(size_t)item * a.dout_stride + r] = dsh[r] == 0.0 ? 1.0 : dsh[r];
 		if (a.pvt) a.pvt[(size_t)item * a.p_stride + r] = pvt[r];
@@ -664,19 +695,14 @@ __global__ void __maxnreg__(96) k_qrp(QrArgs<T> a)
 	__shared__ int s_bi[NW];
 	bool nan_seen = false;
 	const T *X = a.X + (size_t)item * a.x_stride;
-	if (a.trans) {
-		for (int c = w; c < N; c += NW)
-			for (int r = lane; r < N; r += 32) A[c + (size_t)ld * r] = conjv(X[r + (size_t)N * c]);
-		__syncthreads();
-	}
 	{
 		double best = -1.0;
 		int bi = N;
 		for (int c = w; c < N; c += NW) {
 			double s = 0.0;
 			for (int r = lane; r < N; r += 32) {
-				const T v = a.trans ? A[r + (size_t)ld * c] : X[r + (size_t)N * c];
-				if (!a.trans) A[r + (size_t)ld * c] = v;
+				const T v = X[r + (size_t)N * c];
+				A[r + (size_t)ld * c] = v;
 				s += abs2(v);
 			}
 			s = sqrt(warp_sum(s));

@@ -68,7 +68,17 @@ static int launch_gemm_cfg(const GemmArgs<T> &g, cudaStream_t st)
 	}
 }
 
-// tile choice: least padded area, larger tiles on ties
+// Tile choice.  A launch that leaves SMs idle is bound by one CTA's chain
+// (launch, first TMA round trip, K in steps), so few matrices take the smallest
+// tiles, whose CTAs have one 8 x 8 DMMA per warp and step: us a launch in a
+// graph, 16 / 32 / 48-64 tiles, real: N = 64 x 2 2.5 / 3.6 / 6.6, N = 144 x 2
+// 3.8 / 5.6 / 9.5, x 16 8.7 / 7.1 / 9.6, x 64 21.7 / 20.7 / 16.3; complex
+// N = 100 x 2 4.8 / 8.8 / 19.3, x 32 15.4 / 18.6 / 19.4.  The lines lie where
+// the next tile overtakes: about 1000 CTAs of 16 x 16 (complex 1600), 600 of
+// 32 x 32 (real).  Beyond, the least padded area counts, larger tiles on ties; the 56
+// and 40 tiles (one warp per 8 columns) are for the sizes between 64 and 48:
+// N = 100 x 512 53.5 us (64: 69.7), N = 196 x 512 260 (32: 346), N = 75 x 512
+// 30.9 (48: 35.9), complex N = 100 x 128 57.4 (64: 65.6).
 template <typename T>
 int launch_gemm(const GemmArgs<T> &g, cudaStream_t st)
 {
@@ -76,17 +86,32 @@ int launch_gemm(const GemmArgs<T> &g, cudaStream_t st)
 	const bool k_staged = g.mode & (GM_A_DD | GM_B_ROWD | GM_B_GATHER);
 	if ((k_staged && g.K > 512) || g.M < 1 || g.N < 1 || g.K < 1 || g.batch < 1) return DQMC_E_ARG;
 	auto pad = [&](int t) { return (long long)((g.M + t - 1) / t * t) * ((g.N + t - 1) / t * t); };
-	const long long p64 = pad(64), p48 = pad(48), p32 = pad(32);
+	int best = 64;
+	for (int t : {56, 48, 40, 32})
+		if (pad(t) < pad(best)) best = t;
+	auto ctas = [&](int t) { return (long long)g.batch * ((g.M + t - 1) / t) * ((g.N + t - 1) / t); };
+	if (ctas(16) <= (is_cplx<T>::value ? 1600 : 1024)) best = 16;
+	else if (!is_cplx<T>::value && ctas(32) <= 600) best = 32;
 	if constexpr (is_cplx<T>::value) {
-		if (p64 <= p48 && p64 <= p32) return launch_gemm_cfg<T, 64, 64, 8, 4, 2, 3>(g, st);
-		if (p48 <= p32) return launch_gemm_cfg<T, 48, 48, 8, 2, 2, 3>(g, st);
-		return launch_gemm_cfg<T, 32, 32, 8, 2, 2, 3>(g, st);
+		switch (best) {
+		case 64: return launch_gemm_cfg<T, 64, 64, 8, 4, 2, 3>(g, st);
+		case 56: return launch_gemm_cfg<T, 56, 56, 8, 1, 7, 3>(g, st);
+		case 48: return launch_gemm_cfg<T, 48, 48, 8, 2, 2, 3>(g, st);
+		case 40: return launch_gemm_cfg<T, 40, 40, 8, 1, 5, 3>(g, st);
+		case 16: return launch_gemm_cfg<T, 16, 16, 16, 2, 2, 3>(g, st);
+		default: return launch_gemm_cfg<T, 32, 32, 8, 2, 2, 3>(g, st);
+		}
 	} else {
-		if (p64 <= p48 && p64 <= p32) return launch_gemm_cfg<T, 64, 64, 16, 2, 2, 3>(g, st);
+		switch (best) {
+		case 64: return launch_gemm_cfg<T, 64, 64, 16, 2, 2, 3>(g, st);
+		case 56: return launch_gemm_cfg<T, 56, 56, 8, 1, 7, 3>(g, st);
 		// k-depth 8: 24-28 KB per CTA, 7-8 CTAs per SM (2-5% over k-depth 16
 		// with its 4-5 CTAs at 512 x 144^3)
-		if (p48 <= p32) return launch_gemm_cfg<T, 48, 48, 8, 2, 2, 3>(g, st);
-		return launch_gemm_cfg<T, 32, 32, 16, 2, 2, 4>(g, st);
+		case 48: return launch_gemm_cfg<T, 48, 48, 8, 2, 2, 3>(g, st);
+		case 40: return launch_gemm_cfg<T, 40, 40, 8, 1, 5, 3>(g, st);
+		case 16: return launch_gemm_cfg<T, 16, 16, 32, 2, 2, 3>(g, st);
+		default: return launch_gemm_cfg<T, 32, 32, 16, 2, 2, 4>(g, st);
+		}
 	}
 }
 

@@ -1497,11 +1497,9 @@ struct Group : GroupBase, ProfHook {
 			launch_count++;
 			return 0;
 		};
-		if (h.M <= 64) return go(k_hqr<T, NBK, 2, NW>);
-		if (h.M <= 128) return go(k_hqr<T, NBK, 4, NW>);
-		if (h.M <= 224) return go(k_hqr<T, NBK, 7, NW>);
-		if (h.M <= 320) return go(k_hqr<T, NBK, 10, NW>);
-		return DQMC_E_ARG;
+		// the sizes UneqState admits
+		if (h.M > 320) return DQMC_E_ARG;
+		return go(k_hqr<T, NBK, NW>);
 	}
 
 	// bsofi (greens.c:266-337) of NB block-cyclic matrices of E x E blocks

@@ -49,7 +49,7 @@ struct QrArgs {
 // barriers) and form its block-reflector factor T (larft, forward
 // columnwise); warps 8-15 meanwhile apply the previous panel's block
 // reflector I - V T^H V^H to the trailing columns (one-panel look-ahead), 8
-// columns per warp as FP64 tensor-core (DMMA m8n8k4) tiles in the real case.
+// columns per warp as FP64 tensor-core (DMMA m8n8k4) tiles.
 // Q is then accumulated backwards, block by block, in the same memory.
 // Outputs: Q, D^-1 R in position order (Rs), diag(R) and the order.
 
@@ -76,144 +76,132 @@ __device__ inline T qrb_v(const T *Vp, int ld, int r, int j0, int k, int nb)
 	return (k < nb && rr >= k) ? ((rr == k) ? one<T>() : Vp[r + (size_t)ld * k]) : zero<T>();
 }
 
-// col[j0..N-1] -= V W (V^H col), W = T^H (HERM) or T, one warp, one column
-template <typename T, int NBK, int RPL, bool HERM>
-__device__ inline void qrb_apply(T *col, const T *Vp, int ld, const T *Tp, int N, int j0, int nb,
-		int lane)
+// C layout -> B layout of an 8 x 8 tile: element (row r, col c) sits in lane
+// 4 c + r % 4, k-step r / 4; lane (lq, lr) of the C layout holds row lq, columns
+// 2 lr + e
+template <typename T>
+__device__ inline void tile_c_to_b(const T (&x)[2], T (&b)[2], int lane)
 {
-	T x[RPL], wv[NBK];
+	const int lr = lane & 3, lq = lane >> 2;
 #pragma unroll
-	for (int k = 0; k < NBK; k++) wv[k] = zero<T>();
-#pragma unroll
-	for (int q = 0; q < RPL; q++) {
-		const int r = j0 + lane + 32 * q;
-		x[q] = (r < N) ? col[r] : zero<T>();
-		if (r < N) {
-#pragma unroll
-			for (int k = 0; k < NBK; k++) wv[k] += conjv(qrb_v(Vp, ld, r, j0, k, nb)) * x[q];
-		}
-	}
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-		for (int k = 0; k < NBK; k++) wv[k] += shfl_xor(wv[k], o);
-	T wp[NBK];
-#pragma unroll
-	for (int k = 0; k < NBK; k++) {
-		T s = zero<T>();
-#pragma unroll
-		for (int m = 0; m < NBK; m++) {
-			if (m >= nb) continue;
-			if (HERM) {
-				if (m <= k) s += conjv(Tp[m + NBK * k]) * wv[m];
-			} else {
-				if (m >= k) s += Tp[k + NBK * m] * wv[m];
-			}
-		}
-		wp[k] = s;
-	}
-#pragma unroll
-	for (int q = 0; q < RPL; q++) {
-		const int r = j0 + lane + 32 * q;
-		if (r < N) {
-			T y = x[q];
-#pragma unroll
-			for (int k = 0; k < NBK; k++) y -= qrb_v(Vp, ld, r, j0, k, nb) * wp[k];
-			col[r] = y;
-		}
+	for (int s = 0; s < 2; s++) {
+		const int src = 4 * (4 * s + lr) + (lq >> 1);
+		const T v0 = shfl(x[0], src), v1 = shfl(x[1], src);
+		b[s] = (lq & 1) ? v1 : v0;
 	}
 }
 
-// The same for the 8 real columns c0 .. c0+7 (those < cend) on the FP64
-// tensor cores, one warp: W = V^T C, W' = op(T) W, C -= V W'.  Fragment
-// layouts of m8n8k4: lane l holds A[l/4][l%4], B[l%4][l/4] and
-// C[l/4][2(l%4) + {0,1}]; W moves from the C to the B layout by shuffles.
-template <int NBK, bool HERM>
-__device__ inline void qrb_apply8(double *A, int ld, int c0, int cend, const double *Vp,
-		const double *Tp, int N, int j0, int nb, int lane)
+template <typename T>
+__device__ inline void tile_b_to_c(const T (&b)[2], T (&x)[2], int lane)
 {
-	static_assert(NBK == 8, "one m8n8k4 tile of reflectors");
+	// C lane (lq, lr), element e: row lq, column 2 lr + e, held by B lane
+	// 4 (2 lr + e) + lq % 4 in k-step lq / 4
+	const int lr = lane & 3, lq = lane >> 2;
+#pragma unroll
+	for (int e = 0; e < 2; e++) {
+		const int src = 4 * (2 * lr + e) + (lq & 3);
+		const T v0 = shfl(b[0], src), v1 = shfl(b[1], src);
+		x[e] = (lq < 4) ? v0 : v1;
+	}
+}
+
+// c (8 x 8 accumulators) += a b, one k-step
+__device__ inline void tile_mma(double (&c)[2], double a, double b) { dmma(c[0], c[1], a, b); }
+__device__ inline void tile_mma(zd (&c)[2], zd a, zd b)
+{
+	dmma(c[0].x, c[1].x, a.x, b.x);
+	dmma(c[0].x, c[1].x, -a.y, b.y);
+	dmma(c[0].y, c[1].y, a.x, b.y);
+	dmma(c[0].y, c[1].y, a.y, b.x);
+}
+
+// The block reflector of NBK = 8 reflectors on the 8 columns c0 .. c0+7 (those
+// < cend) on the FP64 tensor cores, one warp: W = V^H C, W' = op(T) W (T^H when
+// HERM), C -= V W'.  v(r, k): V's entry of reflector k at row r; C: element
+// (row r, column c) at C[r + ldc c]; rows r0 .. r1-1.  Fragment layouts of
+// m8n8k4: lane l holds A[l/4][l%4], B[l%4][l/4] and C[l/4][2(l%4) + {0,1}]; W
+// moves from the C to the B layout by shuffles.
+template <typename T, bool HERM, typename V>
+__device__ inline void reflect8(T *C, size_t ldc, int c0, int cend, const V &v, const T *Tp, int r0,
+		int r1, int nb, int lane)
+{
+	constexpr int AC = is_cplx<T>::value ? 2 : 4;   // independent accumulators over row quads
+	constexpr int RT = is_cplx<T>::value ? 2 : 3;   // row tiles at a time
+	constexpr int NBK = 8;
 	const int lr = lane & 3, lq = lane >> 2;
 	const int cb = c0 + lq;
 	const bool cbok = cb < cend;
-	// W: four independent accumulator pairs over row quads r0, r0+4, ...
-	double w[4][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-	for (int r0 = j0; r0 < N; r0 += 16) {
-		double av[4], bv[4];
+	T w[AC][2];
 #pragma unroll
-		for (int u = 0; u < 4; u++) {
-			const int r = r0 + 4 * u + lr;
-			const bool rok = r < N;
-			av[u] = rok ? qrb_v(Vp, ld, r, j0, lq, nb) : 0.0;
-			bv[u] = (rok && cbok) ? A[r + (size_t)ld * cb] : 0.0;
+	for (int u = 0; u < AC; u++) w[u][0] = w[u][1] = zero<T>();
+#pragma unroll 2
+	for (int r = r0; r < r1; r += 4 * AC) {
+		T av[AC], bv[AC];
+#pragma unroll
+		for (int u = 0; u < AC; u++) {
+			const int q = r + 4 * u + lr;
+			const bool ok = q < r1;
+			av[u] = ok ? conjv(v(q, lq)) : zero<T>();
+			bv[u] = (ok && cbok) ? C[q + ldc * cb] : zero<T>();
 		}
 #pragma unroll
-		for (int u = 0; u < 4; u++) dmma(w[u][0], w[u][1], av[u], bv[u]);
+		for (int u = 0; u < AC; u++) tile_mma(w[u], av[u], bv[u]);
 	}
-	const double w0 = (w[0][0] + w[1][0]) + (w[2][0] + w[3][0]);
-	const double w1 = (w[0][1] + w[1][1]) + (w[2][1] + w[3][1]);
-	double u0 = 0.0, u1 = 0.0;
+#pragma unroll
+	for (int u = AC / 2; u > 0; u /= 2)
+#pragma unroll
+		for (int k = 0; k < u; k++)
+#pragma unroll
+			for (int e = 0; e < 2; e++) w[k][e] += w[k + u][e];
+	T b[2], x[2] = {zero<T>(), zero<T>()};
+	tile_c_to_b(w[0], b, lane);
 #pragma unroll
 	for (int s = 0; s < 2; s++) {
-		const int kk = 4 * s + lr, src = 4 * kk + (lq >> 1);
-		const double v0 = __shfl_sync(0xffffffffu, w0, src), v1 = __shfl_sync(0xffffffffu, w1, src);
-		const double b = (lq & 1) ? v1 : v0;
-		double a;
-		if (HERM) a = (kk <= lq && lq < nb) ? Tp[kk + NBK * lq] : 0.0;
-		else a = (lq <= kk && kk < nb) ? Tp[lq + NBK * kk] : 0.0;
-		dmma(u0, u1, a, b);
+		const int kk = 4 * s + lr;
+		T a;
+		if (HERM) a = (kk <= lq && lq < nb) ? conjv(Tp[kk + NBK * lq]) : zero<T>();
+		else a = (lq <= kk && kk < nb) ? Tp[lq + NBK * kk] : zero<T>();
+		tile_mma(x, a, b[s]);
 	}
-	double bw[2];
-#pragma unroll
-	for (int s = 0; s < 2; s++) {
-		const int kk = 4 * s + lr, src = 4 * kk + (lq >> 1);
-		const double v0 = __shfl_sync(0xffffffffu, u0, src), v1 = __shfl_sync(0xffffffffu, u1, src);
-		bw[s] = -((lq & 1) ? v1 : v0);
-	}
-	// C -= V W', three row tiles of 8 at a time
+	tile_c_to_b(x, b, lane);
+	b[0] = -b[0];
+	b[1] = -b[1];
 	const int cc = c0 + 2 * lr;
-	const bool ok0 = cc < cend, ok1 = cc + 1 < cend;
-	for (int r0 = j0; r0 < N; r0 += 24) {
-		double x0[3], x1[3], va[3][2];
+	for (int r = r0; r < r1; r += 8 * RT) {
+		T y[RT][2], va[RT][2];
 #pragma unroll
-		for (int u = 0; u < 3; u++) {
-			const int r = r0 + 8 * u + lq;
-			const bool rok = r < N;
-			const double *p0 = A + r + (size_t)ld * cc;
-			x0[u] = (rok && ok0) ? p0[0] : 0.0;
-			x1[u] = (rok && ok1) ? p0[ld] : 0.0;
+		for (int u = 0; u < RT; u++) {
+			const int q = r + 8 * u + lq;
+			const bool ok = q < r1;
 #pragma unroll
-			for (int s = 0; s < 2; s++) va[u][s] = rok ? qrb_v(Vp, ld, r, j0, 4 * s + lr, nb) : 0.0;
+			for (int e = 0; e < 2; e++) y[u][e] = (ok && cc + e < cend) ? C[q + ldc * (cc + e)] : zero<T>();
+#pragma unroll
+			for (int s = 0; s < 2; s++) va[u][s] = ok ? v(q, 4 * s + lr) : zero<T>();
 		}
 #pragma unroll
 		for (int s = 0; s < 2; s++)
 #pragma unroll
-			for (int u = 0; u < 3; u++) dmma(x0[u], x1[u], va[u][s], bw[s]);
+			for (int u = 0; u < RT; u++) tile_mma(y[u], va[u][s], b[s]);
 #pragma unroll
-		for (int u = 0; u < 3; u++) {
-			const int r = r0 + 8 * u + lq;
-			if (r < N) {
-				double *p0 = A + r + (size_t)ld * cc;
-				if (ok0) p0[0] = x0[u];
-				if (ok1) p0[ld] = x1[u];
-			}
+		for (int u = 0; u < RT; u++) {
+			const int q = r + 8 * u + lq;
+#pragma unroll
+			for (int e = 0; e < 2; e++)
+				if (q < r1 && cc + e < cend) C[q + ldc * (cc + e)] = y[u][e];
 		}
 	}
 }
 
-// columns [cfirst, N) in groups of 8 (real, tensor cores) or one by one
-// (complex), group g taken by warp `slot` when g % nslots == slot
-template <typename T, int NBK, int RPL, bool HERM>
-__device__ inline void qrb_apply_cols(T *A, int ld, int cfirst, const T *Vp, const T *Tp, int N,
-		int j0, int nb, int slot, int nslots, int lane)
+// columns [cfirst, N) in groups of 8, group g taken by warp `slot` when
+// g % nslots == slot
+template <typename T, int NBK, bool HERM>
+__device__ inline void qrb_apply_cols(T *A, int ld, int cfirst, int cend, const T *Vp, const T *Tp,
+		int N, int j0, int nb, int slot, int nslots, int lane)
 {
-	if constexpr (is_cplx<T>::value) {
-		for (int c = cfirst + slot; c < N; c += nslots)
-			qrb_apply<T, NBK, RPL, HERM>(A + (size_t)ld * c, Vp, ld, Tp, N, j0, nb, lane);
-	} else {
-		for (int c = cfirst + 8 * slot; c < N; c += 8 * nslots)
-			qrb_apply8<NBK, HERM>(A, ld, c, N, Vp, Tp, N, j0, nb, lane);
-	}
+	static_assert(NBK == 8, "one m8n8k4 tile of reflectors");
+	for (int c = cfirst + 8 * slot; c < cend; c += 8 * nslots)
+		reflect8<T, HERM>(A, (size_t)ld, c, cend, [&](int r, int k) { return qrb_v(Vp, ld, r, j0, k, nb); }, Tp,
+		                  j0, N, nb, lane);
 }
 
 // T of the block of reflectors j0 .. j0+nb-1 stored below the diagonal of
@@ -280,8 +268,7 @@ __device__ inline void qrb_form_q(const QrArgs<T> &a, int item, T *A, int ld, T 
 			A[j0 + q - c * nb + (size_t)ld * (j1 + c)] = zero<T>();
 		}
 		__syncthreads();
-		qrb_apply_cols<T, NBK, RPL, false>(A, ld, j0, Vb, Ts + (size_t)p * NBK * NBK, N, j0, nb, w, NW,
-		                                   lane);
+		qrb_apply_cols<T, NBK, false>(A, ld, j0, N, Vb, Ts + (size_t)p * NBK * NBK, N, j0, nb, w, NW, lane);
 		__syncthreads();
 	}
 	T *Q = a.Q + (size_t)item * a.q_stride;
@@ -491,17 +478,12 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 		if (w < NBK) {
 			if (j1 < N) {
 				// the next panel's columns first, then that panel
-				if constexpr (is_cplx<T>::value) {
-					if (j1 + w < N)
-						qrb_apply<T, NBK, RPL, true>(A + (size_t)ld * (j1 + w), Vp, ld, Tp, N, j0, nb, lane);
-				} else {
-					if (w == 0) qrb_apply8<NBK, true>(A, ld, j1, min(j1 + NBK, N), Vp, Tp, N, j0, nb, lane);
-				}
+				qrb_apply_cols<T, NBK, true>(A, ld, j1, min(j1 + NBK, N), Vp, Tp, N, j0, nb, w, NBK, lane);
 				bar_panel();
 				panel(p + 1);
 			}
 		} else {
-			qrb_apply_cols<T, NBK, RPL, true>(A, ld, j1 + NBK, Vp, Tp, N, j0, nb, w - NBK, NW - NBK, lane);
+			qrb_apply_cols<T, NBK, true>(A, ld, j1 + NBK, N, Vp, Tp, N, j0, nb, w - NBK, NW - NBK, lane);
 		}
 		__syncthreads();
 	}
@@ -1078,45 +1060,6 @@ __device__ inline void lu_panel(T *M, int ld, int N, int j0, int pb, int *ipiv, 
 			mv.dst[i] = pos[t];
 		}
 	}
-}
-
-// C layout -> B layout of an 8 x 8 tile: element (row r, col c) sits in lane
-// 4 c + r % 4, k-step r / 4; lane (lq, lr) of the C layout holds row lq, columns
-// 2 lr + e
-template <typename T>
-__device__ inline void tile_c_to_b(const T (&x)[2], T (&b)[2], int lane)
-{
-	const int lr = lane & 3, lq = lane >> 2;
-#pragma unroll
-	for (int s = 0; s < 2; s++) {
-		const int src = 4 * (4 * s + lr) + (lq >> 1);
-		const T v0 = shfl(x[0], src), v1 = shfl(x[1], src);
-		b[s] = (lq & 1) ? v1 : v0;
-	}
-}
-
-template <typename T>
-__device__ inline void tile_b_to_c(const T (&b)[2], T (&x)[2], int lane)
-{
-	// C lane (lq, lr), element e: row lq, column 2 lr + e, held by B lane
-	// 4 (2 lr + e) + lq % 4 in k-step lq / 4
-	const int lr = lane & 3, lq = lane >> 2;
-#pragma unroll
-	for (int e = 0; e < 2; e++) {
-		const int src = 4 * (2 * lr + e) + (lq & 3);
-		const T v0 = shfl(b[0], src), v1 = shfl(b[1], src);
-		x[e] = (lq < 4) ? v0 : v1;
-	}
-}
-
-// c (8 x 8 accumulators) += a b, one k-step
-__device__ inline void tile_mma(double (&c)[2], double a, double b) { dmma(c[0], c[1], a, b); }
-__device__ inline void tile_mma(zd (&c)[2], zd a, zd b)
-{
-	dmma(c[0].x, c[1].x, a.x, b.x);
-	dmma(c[0].x, c[1].x, -a.y, b.y);
-	dmma(c[0].y, c[1].y, a.x, b.y);
-	dmma(c[0].y, c[1].y, a.y, b.x);
 }
 
 // the rows j0 .. j0+pb-1 of U in the columns c0 .. c0+7 (those < N) right of

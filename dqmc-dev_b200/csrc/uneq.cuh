@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "gemm.cuh"
+#include "qr.cuh"
 
 namespace dq {
 
@@ -83,8 +84,13 @@ __global__ void k_add_diag(int n, int NB, T *A, long long s)
 // (rows of the panel).  The reflectors are LAPACK's geqrf convention
 // (zgeqr2/zlarfg: beta = -sign(Re alpha) ||x||); NBK of them at a time are
 // factored in shared memory and applied to the trailing columns as one
-// block reflector I - V T^H V^H (larft forward, columnwise), so every
-// trailing column is read and written once per block.
+// block reflector I - V T^H V^H (larft forward, columnwise), 8 columns per warp
+// by DMMA (reflect8), so every trailing column is read twice and written once
+// per block.
+// Bound by latency: one CTA per item, M / 8 panels in series.  8x8, four sweeps
+// with unequal-time of one chain: 23.7 -> 23.0 ms; complex 10x10 x 64, with
+// k_qrb's complex panels through the same tiles: 98.6 -> 87.9 ms a sweep (k_qrb
+// 17 -> 12.2 ms of it), before: one column per warp.
 
 template <typename T>
 struct HqrArgs {
@@ -102,7 +108,7 @@ size_t hqr_smem_bytes(int M)
 	return sizeof(T) * ((size_t)M * NBK + NBK * NBK + NBK) + sizeof(double) * NW + 64;
 }
 
-template <typename T, int NBK, int MAXR, int NW>
+template <typename T, int NBK, int NW>
 __global__ void __launch_bounds__(NW * 32) k_hqr(HqrArgs<T> a)
 {
 	const int item = blockIdx.x;
@@ -117,7 +123,7 @@ __global__ void __launch_bounds__(NW * 32) k_hqr(HqrArgs<T> a)
 	T *A = a.A + a.aA.off(item);
 	T *Q = a.Qh + a.aQ.off(item);
 	T *X2 = a.nx2 ? a.X + a.aX.off(item) : nullptr;
-	if (M > 32 * MAXR || n > M) {
+	if (n > M) {
 		if (tid == 0) atomicOr(a.err, DQ_ERR_SIZE);
 		return;
 	}
@@ -215,60 +221,19 @@ __global__ void __launch_bounds__(NW * 32) k_hqr(HqrArgs<T> a)
 			}
 		}
 		__syncthreads();
-		// trailing columns: col -= V T^H (V^H col), rows j0..M-1
-		const int nA = n - j0 - nb;
-		const int ntot = nA + a.nx1 + a.nx2 + M;
-		for (int t = w; t < ntot; t += NW) {
-			T *col;
-			if (t < nA) col = A + (size_t)lda * (j0 + nb + t);
-			else if (t < nA + a.nx1) col = A + (size_t)lda * (n + t - nA);
-			else if (t < nA + a.nx1 + a.nx2) col = X2 + (size_t)lda * (t - nA - a.nx1);
-			else col = Q + (size_t)M * (t - nA - a.nx1 - a.nx2);
-			T x[MAXR], wv[NBK];
-#pragma unroll
-			for (int k = 0; k < NBK; k++) wv[k] = zero<T>();
-#pragma unroll
-			for (int p = 0; p < MAXR; p++) {
-				const int r = lane + 32 * p;
-				x[p] = (r < mr) ? col[j0 + r] : zero<T>();
-				if (r < mr) {
-#pragma unroll
-					for (int k = 0; k < NBK; k++) {
-						if (k < nb && r >= k) {
-							const T v = (r == k) ? one<T>() : V[r + (size_t)M * k];
-							wv[k] += conjv(v) * x[p];
-						}
-					}
-				}
-			}
-#pragma unroll
-			for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-				for (int k = 0; k < NBK; k++) wv[k] += shfl_xor(wv[k], o);
-			T wp[NBK];
-#pragma unroll
-			for (int k = 0; k < NBK; k++) {
-				T s = zero<T>();
-#pragma unroll
-				for (int p = 0; p < NBK; p++)
-					if (p <= k && k < nb) s += conjv(Tt[p + NBK * k]) * wv[p];
-				wp[k] = s;
-			}
-#pragma unroll
-			for (int p = 0; p < MAXR; p++) {
-				const int r = lane + 32 * p;
-				if (r < mr) {
-					T y = x[p];
-#pragma unroll
-					for (int k = 0; k < NBK; k++) {
-						if (k < nb && r >= k) {
-							const T v = (r == k) ? one<T>() : V[r + (size_t)M * k];
-							y -= v * wp[k];
-						}
-					}
-					col[j0 + r] = y;
-				}
-			}
+		// trailing columns: C -= V T^H (V^H C), rows j0..M-1, 8 columns a warp:
+		// those of the panel and the nx1 right of it, X, Q
+		const int n1 = n - j0 - nb + a.nx1, t1 = (n1 + 7) / 8, t2 = (a.nx2 + 7) / 8, t3 = (M + 7) / 8;
+		auto v = [&](int r, int k) {
+			return (k < nb && r >= k) ? ((r == k) ? one<T>() : V[r + (size_t)M * k]) : zero<T>();
+		};
+		for (int t = w; t < t1 + t2 + t3; t += NW) {
+			if (t < t1)
+				reflect8<T, true>(A + j0 + (size_t)lda * (j0 + nb), (size_t)lda, 8 * t, n1, v, Tt, 0, mr, nb, lane);
+			else if (t < t1 + t2)
+				reflect8<T, true>(X2 + j0, (size_t)lda, 8 * (t - t1), a.nx2, v, Tt, 0, mr, nb, lane);
+			else
+				reflect8<T, true>(Q + j0, (size_t)M, 8 * (t - t1 - t2), M, v, Tt, 0, mr, nb, lane);
 		}
 		__syncthreads();
 	}
@@ -476,7 +441,7 @@ struct UePlan {
 template <typename T>
 struct UneqState {
 	// sizes the kernels here take: trtri keeps an N x N block in shared
-	// memory, k_hqr holds 2N rows in MAXR = 10 registers per lane
+	// memory, k_hqr a panel of 2N x 8
 	static bool supported(int N, int F, int L)
 	{
 		const int nmax = is_cplx<T>::value ? 112 : 160;

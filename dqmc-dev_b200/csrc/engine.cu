@@ -1488,7 +1488,7 @@ struct Group : GroupBase, ProfHook {
 	int launch_hqr(const HqrArgs<T> &h)
 	{
 		constexpr int NBK = 8, NW = 16;
-		const size_t sm = hqr_smem_bytes<T, NBK, NW>(h.M);
+		const size_t sm = hqr_smem_bytes<T, NBK>(h.M);
 		auto go = [&](auto kern) -> int {
 			CK(raise_smem(kern, sm));
 			prof_begin(0);
@@ -1497,9 +1497,13 @@ struct Group : GroupBase, ProfHook {
 			launch_count++;
 			return 0;
 		};
-		// the sizes UneqState admits
-		if (h.M > 320) return DQMC_E_ARG;
-		return go(k_hqr<T, NBK, NW>);
+		if (h.M <= 128) return go(k_hqr<T, NBK, NW, 1>);
+		if (h.M <= 256) return go(k_hqr<T, NBK, NW, 2>);
+		if constexpr (!is_cplx<T>::value) {
+			// up to 2 N of the largest N that UneqState admits
+			if (h.M <= 384) return go(k_hqr<T, NBK, NW, 3>);
+		}
+		return DQMC_E_ARG;
 	}
 
 	// bsofi (greens.c:266-337) of NB block-cyclic matrices of E x E blocks

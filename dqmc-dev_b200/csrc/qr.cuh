@@ -45,11 +45,9 @@ struct QrArgs {
 // The QR_PRESORT factorisation (greens.c:119-146: columns scaled by
 // the previous D, ordered by descending norm, then geqrf and the explicit
 // Q), with the matrix in shared memory and the reflectors taken NBK = 8 at
-// a time.  Warps 0-7 factor a panel of 8 columns (one column each, named
-// barriers) and form its block-reflector factor T (larft, forward
-// columnwise); warps 8-15 meanwhile apply the previous panel's block
-// reflector I - V T^H V^H to the trailing columns (one-panel look-ahead), 8
-// columns per warp as FP64 tensor-core (DMMA m8n8k4) tiles.
+// a time.  Warps 0-3 carry the block reflector I - V T^H V^H of a panel to the
+// next panel's columns and factor that panel (qr_panel8); the other 12 take it to
+// the remaining columns meanwhile (reflect8, FP64 tensor-core tiles).
 // Q is then accumulated backwards, block by block, in the same memory.
 // Outputs: Q, D^-1 R in position order (Rs), diag(R) and the order.
 
@@ -64,17 +62,19 @@ template <typename T, int NBK>
 size_t qrb_smem_bytes(int N, bool gm = false)
 {
 	const int np = (N + NBK - 1) / NBK, ld = gm ? N : qrb_ld(N);
-	return sizeof(T) * ((gm ? 0 : (size_t)ld * N) + (size_t)ld * NBK + N + (size_t)np * NBK * NBK)
+	return sizeof(T) * ((gm ? (size_t)ld * NBK : (size_t)ld * N) + (size_t)ld * NBK + N
+	                    + (size_t)np * NBK * NBK)
 	       + sizeof(double) * 3 * (size_t)N + sizeof(int) * (size_t)N + 64;
 }
 
-// reflector k of a panel at global row r (< N): unit diagonal, zero above
-template <typename T>
-__device__ inline T qrb_v(const T *Vp, int ld, int r, int j0, int k, int nb)
-{
-	const int rr = r - j0;
-	return (k < nb && rr >= k) ? ((rr == k) ? one<T>() : Vp[r + (size_t)ld * k]) : zero<T>();
-}
+// warps that factor a panel, and rows of it per lane: two while the panel's
+// rows fit a thread's registers, else four (us a launch of two items, with one /
+// two / four warps: N = 64 106 / 72 / 72, N = 144 281 / 201 / 205)
+template <typename T, int RPL>
+struct QrbPanel {
+	static constexpr int PW = (!is_cplx<T>::value && RPL <= 5) ? 2 : 4;
+	static constexpr int RP = (RPL + PW - 1) / PW;
+};
 
 // C layout -> B layout of an 8 x 8 tile: element (row r, col c) sits in lane
 // 4 c + r % 4, k-step r / 4; lane (lq, lr) of the C layout holds row lq, columns
@@ -115,37 +115,62 @@ __device__ inline void tile_mma(zd (&c)[2], zd a, zd b)
 	dmma(c[0].y, c[1].y, a.y, b.x);
 }
 
-// The block reflector of NBK = 8 reflectors on the 8 columns c0 .. c0+7 (those
-// < cend) on the FP64 tensor cores, one warp: W = V^H C, W' = op(T) W (T^H when
-// HERM), C -= V W'.  v(r, k): V's entry of reflector k at row r; C: element
-// (row r, column c) at C[r + ldc c]; rows r0 .. r1-1.  Fragment layouts of
-// m8n8k4: lane l holds A[l/4][l%4], B[l%4][l/4] and C[l/4][2(l%4) + {0,1}]; W
-// moves from the C to the B layout by shuffles.
-template <typename T, bool HERM, typename V>
-__device__ inline void reflect8(T *C, size_t ldc, int c0, int cend, const V &v, const T *Tp, int r0,
-		int r1, int nb, int lane)
+// reflector k of a panel at its row r: unit diagonal, zero above; V keeps R there
+template <typename T>
+__device__ inline T qr_v8(const T *V, size_t ldv, int r, int k, int mr, int nb)
 {
-	constexpr int AC = is_cplx<T>::value ? 2 : 4;   // independent accumulators over row quads
-	constexpr int RT = is_cplx<T>::value ? 2 : 3;   // row tiles at a time
-	constexpr int NBK = 8;
+	if (k >= nb || r < k || r >= mr) return zero<T>();
+	return (r == k) ? one<T>() : V[r + ldv * k];
+}
+
+// The block reflector of 8 reflectors on the 8 columns of C (ncol of them
+// present) on the FP64 tensor cores, one warp: W = V^H C, W' = op(T) W (T^H
+// when HERM), C -= V W'.  V and C from the panel's first row on, mr rows; the
+// first 8 rows of V hold R on and above the diagonal (qr_v8), the others
+// are read as they are, so columns k >= nb hold zeros there.  Fragment layouts
+// of m8n8k4: lane l holds A[l/4][l%4], B[l%4][l/4] and C[l/4][2(l%4) + {0,1}];
+// W moves from the C to the B layout by shuffles.  Absent columns are computed
+// on the last present one and not stored.  AC row quads and RT row tiles are in
+// flight at a time, more when C lies in global memory.
+// Bound by the FP64 tensor pipe (16 cycles a DMMA and SM quarter) when all
+// warps have columns, else by the chain load - product - store; the full row
+// groups carry no row or column test, which cost more issue slots than the
+// products.
+template <typename T, bool HERM, int AC, int RT>
+__device__ inline void reflect8(T *C, size_t ldc, int ncol, const T *V, size_t ldv, const T *Tp, int mr,
+		int nb, int lane)
+{
 	const int lr = lane & 3, lq = lane >> 2;
-	const int cb = c0 + lq;
-	const bool cbok = cb < cend;
 	T w[AC][2];
 #pragma unroll
 	for (int u = 0; u < AC; u++) w[u][0] = w[u][1] = zero<T>();
+	const T *cb = C + ldc * min(lq, ncol - 1), *vb = V + ldv * lq;
+	{
+		T av[2], bv[2];
+#pragma unroll
+		for (int u = 0; u < 2; u++) {
+			const int q = 4 * u + lr;
+			av[u] = conjv(qr_v8(V, ldv, q, lq, mr, nb));
+			bv[u] = q < mr ? cb[q] : zero<T>();
+		}
+#pragma unroll
+		for (int u = 0; u < 2; u++) tile_mma(w[u % AC], av[u], bv[u]);
+	}
+	int r = 8;
 #pragma unroll 2
-	for (int r = r0; r < r1; r += 4 * AC) {
+	for (; r + 4 * AC <= mr; r += 4 * AC) {
 		T av[AC], bv[AC];
 #pragma unroll
 		for (int u = 0; u < AC; u++) {
-			const int q = r + 4 * u + lr;
-			const bool ok = q < r1;
-			av[u] = ok ? conjv(v(q, lq)) : zero<T>();
-			bv[u] = (ok && cbok) ? C[q + ldc * cb] : zero<T>();
+			av[u] = conjv(vb[r + 4 * u + lr]);
+			bv[u] = cb[r + 4 * u + lr];
 		}
 #pragma unroll
 		for (int u = 0; u < AC; u++) tile_mma(w[u], av[u], bv[u]);
+	}
+	for (; r < mr; r += 4) {
+		const bool ok = r + lr < mr;
+		tile_mma(w[0], ok ? conjv(vb[r + lr]) : zero<T>(), ok ? cb[r + lr] : zero<T>());
 	}
 #pragma unroll
 	for (int u = AC / 2; u > 0; u /= 2)
@@ -159,49 +184,317 @@ __device__ inline void reflect8(T *C, size_t ldc, int c0, int cend, const V &v, 
 	for (int s = 0; s < 2; s++) {
 		const int kk = 4 * s + lr;
 		T a;
-		if (HERM) a = (kk <= lq && lq < nb) ? conjv(Tp[kk + NBK * lq]) : zero<T>();
-		else a = (lq <= kk && kk < nb) ? Tp[lq + NBK * kk] : zero<T>();
+		if (HERM) a = (kk <= lq && lq < nb) ? conjv(Tp[kk + 8 * lq]) : zero<T>();
+		else a = (lq <= kk && kk < nb) ? Tp[lq + 8 * kk] : zero<T>();
 		tile_mma(x, a, b[s]);
 	}
 	tile_c_to_b(x, b, lane);
 	b[0] = -b[0];
 	b[1] = -b[1];
-	const int cc = c0 + 2 * lr;
-	for (int r = r0; r < r1; r += 8 * RT) {
+	const bool st[2] = {2 * lr < ncol, 2 * lr + 1 < ncol};
+	T *ce[2] = {C + ldc * min(2 * lr, ncol - 1) + lq, C + ldc * min(2 * lr + 1, ncol - 1) + lq};
+	const T *vs[2] = {V + ldv * lr + lq, V + ldv * (4 + lr) + lq};
+	// one row tile with every test
+	auto edge = [&](int r, bool top) {
+		const bool ok = r + lq < mr;
+		T y[2];
+#pragma unroll
+		for (int e = 0; e < 2; e++) y[e] = ok ? ce[e][r] : zero<T>();
+#pragma unroll
+		for (int s = 0; s < 2; s++)
+			tile_mma(y, top ? qr_v8(V, ldv, lq, 4 * s + lr, mr, nb) : (ok ? vs[s][r] : zero<T>()), b[s]);
+#pragma unroll
+		for (int e = 0; e < 2; e++)
+			if (ok && st[e]) ce[e][r] = y[e];
+	};
+	edge(0, true);
+	r = 8;
+	for (; r + 8 * RT <= mr; r += 8 * RT) {
 		T y[RT][2], va[RT][2];
 #pragma unroll
-		for (int u = 0; u < RT; u++) {
-			const int q = r + 8 * u + lq;
-			const bool ok = q < r1;
+		for (int u = 0; u < RT; u++)
 #pragma unroll
-			for (int e = 0; e < 2; e++) y[u][e] = (ok && cc + e < cend) ? C[q + ldc * (cc + e)] : zero<T>();
-#pragma unroll
-			for (int s = 0; s < 2; s++) va[u][s] = ok ? v(q, 4 * s + lr) : zero<T>();
-		}
+			for (int e = 0; e < 2; e++) {
+				y[u][e] = ce[e][r + 8 * u];
+				va[u][e] = vs[e][r + 8 * u];
+			}
 #pragma unroll
 		for (int s = 0; s < 2; s++)
 #pragma unroll
 			for (int u = 0; u < RT; u++) tile_mma(y[u], va[u][s], b[s]);
 #pragma unroll
-		for (int u = 0; u < RT; u++) {
-			const int q = r + 8 * u + lq;
+		for (int u = 0; u < RT; u++)
 #pragma unroll
 			for (int e = 0; e < 2; e++)
-				if (q < r1 && cc + e < cend) C[q + ldc * (cc + e)] = y[u][e];
+				if (st[e]) ce[e][r + 8 * u] = y[u][e];
+	}
+	for (; r < mr; r += 8) edge(r, false);
+}
+
+// depths of reflect8 for columns in shared and in global memory
+template <typename T, bool GMEM>
+struct ReflectDepth {
+	static constexpr int AC = is_cplx<T>::value ? (GMEM ? 4 : 2) : (GMEM ? 8 : 4);
+	static constexpr int RT = is_cplx<T>::value ? (GMEM ? 4 : 2) : (GMEM ? 8 : 3);
+};
+
+// depths of reflect_next for up to 32 RPL rows
+template <typename T, int RPL>
+struct NextDepth {
+	static constexpr int AC = is_cplx<T>::value ? (RPL > 2 ? 4 : 2) : (RPL > 4 ? 8 : RPL > 1 ? 4 : 2);
+	static constexpr int RT = is_cplx<T>::value ? (RPL < 3 ? RPL : 3) : (RPL < 6 ? RPL : (RPL + 1) / 2);
+};
+
+// columns [cfirst, cend) of A in groups of 8, group g taken by warp `slot` when
+// g % nslots == slot; Vp and A from row j0 on
+template <typename T, bool HERM, bool GMEM>
+__device__ inline void reflect_cols(T *A, size_t lda, int cfirst, int cend, const T *Vp, size_t ldv,
+		const T *Tp, int mr, int nb, int slot, int nslots, int lane)
+{
+	using D = ReflectDepth<T, GMEM>;
+	for (int c = cfirst + 8 * slot; c < cend; c += 8 * nslots)
+		reflect8<T, HERM, D::AC, D::RT>(A + lda * c, lda, min(8, cend - c), Vp, ldv, Tp, mr, nb, lane);
+}
+
+// ----------------------------------------------- panel of 8 columns
+//
+// Householder QR of mr x nb (nb <= 8) by PW warps, each lane holding its rows
+// lane + 32 (w + PW t), t < RP, of all 8 columns in registers, and the block's
+// T (larft, forward columnwise).  Per reflector k one reduction gives
+// x_k^H x_c below row k for every column c: the norm (c = k), v_k^H x_c of the
+// later columns and v_c^H v_k of the earlier ones, with v_k = scal x_k below the
+// diagonal and 1 on it (zlarfg convention).  The 8 sums are folded onto the
+// lanes, lane 4 s + {0..3} ending up with slot s, and each lane forms its
+// slot's coefficient: one barrier per reflector and no second reduction.  Bound
+// by that chain of latencies (about 1000 cycles a reflector, 300 of them the
+// square root and the division), so
+// - the columns rotate through the slots and the loop is not unrolled,
+// - the odd lanes divide by beta while the even ones divide by the pivot, and
+// - T is solved for at the end, one column a lane.
+// One column per warp with two barriers and two reductions per reflector before:
+// k_qrb 275 -> 201 us at N = 144 x 2, 1050 -> 800 us at N = 144 x 512, complex
+// N = 100 x 64 320 -> 238 us, with the products of reflect8.
+// load(r, c): the panel's entries; store(r, c, v) for all 8 columns: R on and
+// above the diagonal, V below, zero for c >= nb.
+template <typename T, int PW>
+struct PanelShared {
+	T red[2][PW][8], xrow[2][8], scal[PW][8], g[PW][8], y[8][8];
+	T wred[4][64];
+};
+
+template <int NWARP>
+__device__ inline void bar_panel()
+{
+	asm volatile("barrier.sync 1, %0;\n" ::"n"(NWARP * 32) : "memory");
+}
+
+template <typename T, int PW, int RP, typename L, typename S>
+__device__ inline void qr_panel8(PanelShared<T, PW> &sh, int mr, int nb, int w, int lane, T *Tp, T *tau,
+		double *beta_out, double *vv, const L &load, const S &store)
+{
+	const int r0 = lane + 32 * w, cl = lane >> 2;
+	if (nb < 8 && w == PW - 1) sh.y[lane >> 3][lane & 7] = sh.y[4 + (lane >> 3)][lane & 7] = zero<T>();
+	T x[8][RP];
+#pragma unroll
+	for (int c = 0; c < 8; c++)
+#pragma unroll
+		for (int t = 0; t < RP; t++) {
+			const int r = r0 + 32 * PW * t;
+			x[c][t] = (c < nb && r < mr) ? load(r, c) : zero<T>();
+		}
+	// slot s holds column (k + s) mod 8
+	auto rotate = [&]() {
+#pragma unroll
+		for (int t = 0; t < RP; t++) {
+			const T first = x[0][t];
+#pragma unroll
+			for (int s = 0; s < 7; s++) x[s][t] = x[s + 1][t];
+			x[7][t] = first;
+		}
+	};
+#pragma unroll 1
+	for (int k = 0; k < nb; k++) {
+		T *xr = sh.xrow[k & 1];
+		if (r0 == k) {
+#pragma unroll
+			for (int s = 0; s < 8; s++) xr[s] = x[s][0];
+		}
+		T d[8];
+#pragma unroll
+		for (int s = 0; s < 8; s++) d[s] = zero<T>();
+#pragma unroll
+		for (int t = 0; t < RP; t++) {
+			const T xk = (t == 0 && r0 <= k) ? zero<T>() : conjv(x[0][t]);
+#pragma unroll
+			for (int s = 0; s < 8; s++) d[s] += xk * x[s][t];
+		}
+#pragma unroll
+		for (int o = 16, n = 4; n > 0; o >>= 1, n >>= 1) {
+			const bool up = lane & o;
+#pragma unroll
+			for (int i = 0; i < n; i++) {
+				const T send = up ? d[i] : d[i + n];
+				d[i] = (up ? d[i + n] : d[i]) + shfl_xor(send, o);
+			}
+		}
+		T sm = d[0];
+		sm += shfl_xor(sm, 2);
+		sm += shfl_xor(sm, 1);
+		double sig;
+		if (PW > 1) {
+			if ((lane & 3) == 0) sh.red[k & 1][w][cl] = sm;
+			bar_panel<PW>();
+			sm = sh.red[k & 1][0][cl];
+			sig = re(sh.red[k & 1][0][0]);
+#pragma unroll
+			for (int q = 1; q < PW; q++) {
+				sm += sh.red[k & 1][q][cl];
+				sig += re(sh.red[k & 1][q][0]);
+			}
+		} else {
+			__syncwarp();
+			sig = re(shfl(sm, 0));
+		}
+		const T alpha = xr[0], xc = xr[cl], sy = sh.scal[w][(k + cl) & 7];
+		const bool none = sig == 0.0 && im(alpha) == 0.0;
+		const double beta = none ? re(alpha) : -copysign(sqrt(abs2(alpha) + sig), re(alpha));
+		const T del = alpha - beta;
+		const double den = (lane & 1) ? beta : (is_cplx<T>::value ? abs2(del) : re(del));
+		const double iq = 1.0 / den, io = __shfl_xor_sync(0xffffffffu, iq, 1);
+		const double ib = (lane & 1) ? iq : io, ia = (lane & 1) ? io : iq;
+		T scal = is_cplx<T>::value ? conjv(del) * ia : from_re<T>(ia), tk = -(del * ib), sb = scal * ib;
+		if (none) scal = tk = sb = zero<T>();
+		// later columns: x_c -= u g, u = x_k with alpha - beta on the diagonal (v_k / scal)
+		const T g = (cl > 0 && cl < 8 - k) ? -((conjv(del) * xc + sm) * sb) : zero<T>();
+		if ((lane & 3) == 0) sh.g[w][cl] = g;
+		__syncwarp();
+		if (r0 == k) x[0][0] = del;
+		T u[RP];
+#pragma unroll
+		for (int t = 0; t < RP; t++) u[t] = (t == 0 && r0 < k) ? zero<T>() : x[0][t];
+#pragma unroll
+		for (int s = 1; s < 8; s++) {
+			const T gs = sh.g[w][s];
+#pragma unroll
+			for (int t = 0; t < RP; t++) x[s][t] -= u[t] * gs;
+		}
+		if (lane == 0) sh.scal[w][k] = scal;
+		if (w == PW - 1) {
+			// earlier ones (unscaled in the registers): y = v_c^H v_k
+			if (lane == 0) {
+				tau[k] = tk;
+				beta_out[k] = beta;
+				vv[k] = 1.0 + sig * abs2(scal);
+			}
+			const T y = conjv(sy) * (scal * (conjv(xc) * del + conjv(sm)));
+			if (cl >= 8 - k && (lane & 3) == 0) sh.y[k + cl - 8][k] = y;
+		}
+		rotate();
+	}
+	for (int k = nb; k < 8; k++) rotate();
+	__syncwarp();
+	if (PW > 1) bar_panel<PW>();
+	if (w == PW - 1 && lane < nb) {
+		// column `lane` of T upwards from its diagonal:
+		// T[i, c] = -tau_i (y_i,i+1 T[i+1, c] + ... + y_ic T[c, c])
+		T tc[8];
+#pragma unroll
+		for (int i = 7; i >= 0; i--) {
+			T ts = zero<T>();
+#pragma unroll
+			for (int m = 7; m > i; m--) ts += sh.y[i][m] * tc[m];
+			const T ti = i < nb ? tau[i] : zero<T>();
+			tc[i] = (i > lane) ? zero<T>() : (i == lane) ? ti : -(ti * ts);
+			if (i <= lane) Tp[i + 8 * lane] = tc[i];
+		}
+	}
+#pragma unroll
+	for (int c = 0; c < 8; c++) {
+		const T sc = c < nb ? sh.scal[w][c] : zero<T>();
+		const double bc = c < nb ? beta_out[c] : 0.0;
+#pragma unroll
+		for (int t = 0; t < RP; t++) {
+			const int r = r0 + 32 * PW * t;
+			T v = x[c][t] * sc;
+			if (t == 0 && r0 <= c) v = (r0 < c) ? x[c][0] : from_re<T>(bc);
+			if (r < mr) store(r, c, v);
 		}
 	}
 }
 
-// columns [cfirst, N) in groups of 8, group g taken by warp `slot` when
-// g % nslots == slot
-template <typename T, int NBK, bool HERM>
-__device__ inline void qrb_apply_cols(T *A, int ld, int cfirst, int cend, const T *Vp, const T *Tp,
-		int N, int j0, int nb, int slot, int nslots, int lane)
+// the block reflector (V, Tp) on the next panel's columns (ncol <= 8), the rows
+// over GW warps; C(r, c) is read through load, written through store
+template <typename T, int GW, int AC, int RT, int PW, typename L, typename S>
+__device__ inline void reflect_next(PanelShared<T, PW> &sh, int ncol, const T *V, size_t ldv, const T *Tp,
+		int mr, int nb, int w, int lane, const L &load, const S &store)
 {
-	static_assert(NBK == 8, "one m8n8k4 tile of reflectors");
-	for (int c = cfirst + 8 * slot; c < cend; c += 8 * nslots)
-		reflect8<T, HERM>(A, (size_t)ld, c, cend, [&](int r, int k) { return qrb_v(Vp, ld, r, j0, k, nb); }, Tp,
-		                  j0, N, nb, lane);
+	const int lr = lane & 3, lq = lane >> 2;
+	T wv[AC][2];
+#pragma unroll
+	for (int u = 0; u < AC; u++) wv[u][0] = wv[u][1] = zero<T>();
+	const int cb = min(lq, ncol - 1);
+	const T *vb = V + ldv * lq;
+	for (int r = 4 * w; r < mr; r += 4 * GW * AC) {
+		T av[AC], bv[AC];
+#pragma unroll
+		for (int u = 0; u < AC; u++) {
+			const int q = r + 4 * GW * u + lr;
+			bv[u] = q < mr ? load(q, cb) : zero<T>();
+			av[u] = q < mr ? conjv(vb[q]) : zero<T>();
+		}
+		if (r < 8) av[0] = conjv(qr_v8(V, ldv, r + lr, lq, mr, nb));
+#pragma unroll
+		for (int u = 0; u < AC; u++) tile_mma(wv[u], av[u], bv[u]);
+	}
+#pragma unroll
+	for (int u = AC / 2; u > 0; u /= 2)
+#pragma unroll
+		for (int k = 0; k < u; k++)
+#pragma unroll
+			for (int e = 0; e < 2; e++) wv[k][e] += wv[k + u][e];
+	sh.wred[w][8 * lq + 2 * lr] = wv[0][0];
+	sh.wred[w][8 * lq + 2 * lr + 1] = wv[0][1];
+	bar_panel<GW>();
+	T y[2] = {zero<T>(), zero<T>()}, b[2];
+#pragma unroll
+	for (int h = 0; h < 2; h++) {
+		const int kk = 4 * h + lr;
+		T bs = sh.wred[0][8 * kk + lq];
+#pragma unroll
+		for (int q = 1; q < GW; q++) bs += sh.wred[q][8 * kk + lq];
+		tile_mma(y, (kk <= lq && lq < nb) ? conjv(Tp[kk + 8 * lq]) : zero<T>(), bs);
+	}
+	tile_c_to_b(y, b, lane);
+	b[0] = -b[0];
+	b[1] = -b[1];
+	const int c0 = min(2 * lr, ncol - 1), c1 = min(2 * lr + 1, ncol - 1);
+	for (int r = 8 * w; r < mr; r += 8 * GW * RT) {
+		T z[RT][2], va[RT][2];
+#pragma unroll
+		for (int u = 0; u < RT; u++) {
+			const int q = r + 8 * GW * u + lq;
+			const bool ok = q < mr;
+			z[u][0] = ok ? load(q, c0) : zero<T>();
+			z[u][1] = ok ? load(q, c1) : zero<T>();
+#pragma unroll
+			for (int h = 0; h < 2; h++) va[u][h] = ok ? V[q + ldv * (4 * h + lr)] : zero<T>();
+		}
+		if (r == 0) {
+#pragma unroll
+			for (int h = 0; h < 2; h++) va[0][h] = qr_v8(V, ldv, lq, 4 * h + lr, mr, nb);
+		}
+#pragma unroll
+		for (int h = 0; h < 2; h++)
+#pragma unroll
+			for (int u = 0; u < RT; u++) tile_mma(z[u], va[u][h], b[h]);
+#pragma unroll
+		for (int u = 0; u < RT; u++) {
+			const int q = r + 8 * GW * u + lq;
+#pragma unroll
+			for (int e = 0; e < 2; e++)
+				if (q < mr && 2 * lr + e < ncol) store(q, 2 * lr + e, z[u][e]);
+		}
+	}
 }
 
 // T of the block of reflectors j0 .. j0+nb-1 stored below the diagonal of
@@ -248,7 +541,7 @@ __device__ inline void qrb_block_t(const T *A, int ld, const T *tau, T *Tp, int 
 // (A second buffer, filled while the previous block is applied, saves the
 // first barrier but takes 9.5 KB more shared memory, which keeps a GEMM CTA
 // of another lane from sharing the SM.)
-template <typename T, int NW, int NBK, int RPL>
+template <typename T, int NW, int NBK, bool GM>
 __device__ inline void qrb_form_q(const QrArgs<T> &a, int item, T *A, int ld, T *Vb, const T *Ts,
 		const T *tau, const double *vv, int N)
 {
@@ -260,7 +553,7 @@ __device__ inline void qrb_form_q(const QrArgs<T> &a, int item, T *A, int ld, T 
 		for (int q = tid; q < nb * mr; q += blockDim.x) {
 			const int k = q / mr, r = j0 + q - k * mr;
 			T *e = A + r + (size_t)ld * (j0 + k);
-			Vb[r + (size_t)ld * k] = *e;
+			Vb[r - j0 + (size_t)ld * k] = *e;
 			*e = (r == j0 + k) ? one<T>() : zero<T>();
 		}
 		for (int q = tid; q < nb * (N - j1); q += blockDim.x) {
@@ -268,16 +561,18 @@ __device__ inline void qrb_form_q(const QrArgs<T> &a, int item, T *A, int ld, T 
 			A[j0 + q - c * nb + (size_t)ld * (j1 + c)] = zero<T>();
 		}
 		__syncthreads();
-		qrb_apply_cols<T, NBK, false>(A, ld, j0, N, Vb, Ts + (size_t)p * NBK * NBK, N, j0, nb, w, NW, lane);
+		reflect_cols<T, false, GM>(A + j0, ld, j0, N, Vb, ld, Ts + (size_t)p * NBK * NBK, mr, nb, w, NW, lane);
 		__syncthreads();
 	}
 	T *Q = a.Q + (size_t)item * a.q_stride;
 	for (int c = w; c < N; c += NW)
 		for (int r = lane; r < N; r += 32) Q[r + (size_t)N * c] = A[r + (size_t)ld * c];
-	if (tid == 0 && a.qdet) {
+	if (w == 0 && a.qdet) {
 		T ph = one<T>();
-		for (int j = 0; j < N; j++) ph = ph * phase_of(one<T>() - tau[j] * vv[j]);
-		a.qdet[item] = ph;
+		for (int j = lane; j < N; j += 32) ph = ph * phase_of(one<T>() - tau[j] * vv[j]);
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) ph = ph * shfl_xor(ph, o);
+		if (lane == 0) a.qdet[item] = ph;
 	}
 }
 
@@ -292,8 +587,9 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 	extern __shared__ __align__(16) unsigned char smraw[];
 	// N columns, leading dimension ld, position order
 	T *A = GM ? a.work + (size_t)item * a.w_stride : (T *)smraw;
-	T *Vb = GM ? (T *)smraw : A + (size_t)ld * N;   // copy of one panel's V (ld x NBK)
-	T *tau = Vb + (size_t)ld * NBK;             // N
+	// copies of a panel's V (ld x NBK): one, in the global-memory form two
+	T *Vb = GM ? (T *)smraw : A + (size_t)ld * N;
+	T *tau = Vb + (GM ? 2 : 1) * (size_t)ld * NBK;   // N
 	T *Ts = tau + N;                            // np blocks of NBK x NBK
 	double *dsh = (double *)(Ts + (size_t)np * NBK * NBK);
 	double *vv = dsh + N;                       // v^H v
@@ -325,10 +621,15 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 			vn[q] = dc ? s * dc[q] * dc[q] : s;
 		}
 	} else {
+#pragma unroll 2
 		for (int c = w; c < N; c += NW) {
 			const double sc = dc ? dc[c] : 1.0;
+			T e[RPL];
+#pragma unroll
+			for (int t = 0; t < RPL; t++) e[t] = lane + 32 * t < N ? X[lane + 32 * t + (size_t)N * c] : zero<T>();
 			double s = 0.0;
-			for (int r = lane; r < N; r += 32) s += abs2(X[r + (size_t)N * c] * sc);
+#pragma unroll
+			for (int t = 0; t < RPL; t++) s += abs2(e[t] * sc);
 			s = warp_sum(s);
 			if (lane == 0) vn[c] = s;
 		}
@@ -343,6 +644,7 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 			if (a.err) atomicOr(a.err, DQ_ERR_NAN);
 		}
 		int rank = 0;
+#pragma unroll 4
 		for (int o = 0; o < N; o++) {
 			double u = vn[o];
 			if (!(u >= 0.0)) u = -1.0;
@@ -358,132 +660,62 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 			for (int c = lane; c < N; c += 32)
 				A[r + (size_t)ld * rk[c]] = conjv(X[c + (size_t)N * r]) * (dc ? dc[c] : 1.0);
 	} else {
+#pragma unroll 2
 		for (int j = w; j < N; j += NW) {
 			const int c = pvt[j];
 			const double sc = dc ? dc[c] : 1.0;
-			for (int r = lane; r < N; r += 32) A[r + (size_t)ld * j] = X[r + (size_t)N * c] * sc;
+			T e[RPL];
+#pragma unroll
+			for (int t = 0; t < RPL; t++) e[t] = lane + 32 * t < N ? X[lane + 32 * t + (size_t)N * c] : zero<T>();
+#pragma unroll
+			for (int t = 0; t < RPL; t++)
+				if (lane + 32 * t < N) A[lane + 32 * t + (size_t)ld * j] = e[t] * sc;
 		}
 	}
 	__syncthreads();
 
-	// panel p by warps 0..NBK-1, warp c holding column j0 + c in registers
-	// (rows j0 + lane + 32 t).  Per reflector k: its owner (warp k) forms it
-	// (zlarfg convention) and publishes v; the later columns' warps update
-	// themselves, the earlier ones give y_c = v_c^H v_k for T (larft); two
-	// named barriers of the panel warps per reflector.  The next owner's
-	// norm below its diagonal is taken in the same pass as its update.
-	static_assert(NW == 2 * NBK, "NBK panel warps and NBK trailing warps");
-	__shared__ T ybuf[NBK];
-	auto bar_panel = []() { asm volatile("barrier.sync 1, %0;\n" ::"r"(NBK * 32) : "memory"); };
+	// Panel p by warps 0..PW-1; then warps 0..GW-1 take its block reflector to
+	// the next panel's columns and factor that panel while the other warps
+	// take it to the rest.  In the global-memory form the next panel and the
+	// reflectors pass through shared memory (two buffers).
+	using ND = NextDepth<T, RPL>;
+	constexpr int PW = QrbPanel<T, RPL>::PW, RP = QrbPanel<T, RPL>::RP, GW = 4;
+	static_assert(NBK == 8 && PW <= GW && GW < NW, "panels of 8 columns, panel warps among the look-ahead's");
+	__shared__ PanelShared<T, PW> sh;
 	auto panel = [&](int p) {
 		const int j0 = p * NBK, nb = min(NBK, N - j0);
-		T *Tp = Ts + (size_t)p * NBK * NBK;
-		const int c = w, jc = j0 + c;
-		T *colc = A + (size_t)ld * jc;
-		T x[RPL];
-#pragma unroll
-		for (int t = 0; t < RPL; t++) {
-			const int r = j0 + lane + 32 * t;
-			x[t] = (c < nb && r < N) ? colc[r] : zero<T>();
-		}
-		double sig = 0.0;
-		if (c == 0) {
-#pragma unroll
-			for (int t = 0; t < RPL; t++)
-				if (j0 + lane + 32 * t > j0) sig += abs2(x[t]);
-			sig = warp_sum(sig);
-		}
-		for (int k = 0; k < nb; k++) {
-			const int j = j0 + k;
-			T tk = zero<T>();
-			if (c == k) {
-				const T alpha = shfl(x[0], k);
-				T scal;
-				double beta;
-				if (sig == 0.0 && im(alpha) == 0.0) {
-					tk = zero<T>();
-					beta = re(alpha);
-					scal = zero<T>();
-				} else {
-					beta = -copysign(sqrt(abs2(alpha) + sig), re(alpha));
-					tk = (from_re<T>(beta) - alpha) / beta;
-					scal = one<T>() / (alpha - beta);
-				}
-#pragma unroll
-				for (int t = 0; t < RPL; t++) {
-					const int r = j0 + lane + 32 * t;
-					if (r > j) x[t] *= scal;
-					else if (r == j) x[t] = from_re<T>(beta);
-					if (r < N) colc[r] = x[t];
-				}
-				if (lane == 0) {
-					tau[j] = tk;
-					dsh[j] = beta;
-					vv[j] = 1.0 + sig * abs2(scal);
-				}
-			}
-			bar_panel();
-			if (c != k && c < nb) {
-				const T *vk = A + (size_t)ld * j;
-				T vr[RPL];
-				T d = zero<T>();
-#pragma unroll
-				for (int t = 0; t < RPL; t++) {
-					const int r = j0 + lane + 32 * t;
-					vr[t] = (r > j && r < N) ? vk[r] : ((r == j) ? one<T>() : zero<T>());
-					d += conjv(vr[t]) * x[t];
-				}
-				d = warp_sum(d);
-				if (c > k) {
-					const T f = conjv(tau[j]) * d;
-					double s2 = 0.0;
-#pragma unroll
-					for (int t = 0; t < RPL; t++) {
-						x[t] -= vr[t] * f;
-						if (j0 + lane + 32 * t > j + 1) s2 += abs2(x[t]);
-					}
-					if (c == k + 1) sig = warp_sum(s2);
-				} else if (lane == 0) {
-					ybuf[c] = conjv(d);
-				}
-			}
-			bar_panel();
-			// T[0:k, k] = -tau_k T[0:k, 0:k] y, T[k, k] = tau_k
-			if (c == k) {
-				if (lane < k) {
-					T sm = zero<T>();
-#pragma unroll
-					for (int m = 0; m < NBK; m++)
-						if (m >= lane && m < k) sm += Tp[lane + NBK * m] * ybuf[m];
-					Tp[lane + NBK * k] = -tk * sm;
-				}
-				if (lane == k) Tp[k + NBK * k] = tk;
-			}
-		}
-		if (c < nb) {
-#pragma unroll
-			for (int t = 0; t < RPL; t++) {
-				const int r = j0 + lane + 32 * t;
-				if (r < N) colc[r] = x[t];
-			}
-		}
+		T *Aj = A + j0 + (size_t)ld * j0;
+		T *Vj = GM ? Vb + (size_t)(p & 1) * ld * NBK : Aj;
+		qr_panel8<T, PW, RP>(
+			sh, N - j0, nb, w, lane, Ts + (size_t)p * NBK * NBK, tau + j0, dsh + j0, vv + j0,
+			[&](int r, int c) { return (GM && p) ? Vj[r + (size_t)ld * c] : Aj[r + (size_t)ld * c]; },
+			[&](int r, int c, T v) {
+				if (c >= nb) return;
+				Aj[r + (size_t)ld * c] = v;
+				if (GM) Vj[r + (size_t)ld * c] = v;
+			});
 	};
-
-	if (w < NBK) panel(0);
+	if (w < PW) panel(0);
 	__syncthreads();
 	for (int p = 0; p < np; p++) {
-		const int j0 = p * NBK, nb = min(NBK, N - j0), j1 = j0 + nb;
-		const T *Vp = A + (size_t)ld * j0;
+		const int j0 = p * NBK, nb = min(NBK, N - j0), j1 = j0 + nb, mr = N - j0;
+		const T *Vp = GM ? Vb + (size_t)(p & 1) * ld * NBK : A + j0 + (size_t)ld * j0;
 		const T *Tp = Ts + (size_t)p * NBK * NBK;
-		if (w < NBK) {
+		if (w < GW) {
 			if (j1 < N) {
-				// the next panel's columns first, then that panel
-				qrb_apply_cols<T, NBK, true>(A, ld, j1, min(j1 + NBK, N), Vp, Tp, N, j0, nb, w, NBK, lane);
-				bar_panel();
-				panel(p + 1);
+				T *C = A + j0 + (size_t)ld * j1, *Vn = Vb + (size_t)((p + 1) & 1) * ld * NBK;
+				reflect_next<T, GW, ND::AC, ND::RT>(
+					sh, min(NBK, N - j1), Vp, ld, Tp, mr, nb, w, lane,
+					[&](int r, int c) { return C[r + (size_t)ld * c]; },
+					[&](int r, int c, T v) {
+						if (GM && r >= NBK) Vn[r - NBK + (size_t)ld * c] = v;
+						else C[r + (size_t)ld * c] = v;
+					});
+				bar_panel<GW>();
+				if (w < PW) panel(p + 1);
 			}
 		} else {
-			qrb_apply_cols<T, NBK, true>(A, ld, j1 + NBK, N, Vp, Tp, N, j0, nb, w - NBK, NW - NBK, lane);
+			reflect_cols<T, true, GM>(A + j0, ld, j1 + NBK, N, Vp, ld, Tp, mr, nb, w - GW, NW - GW, lane);
 		}
 		__syncthreads();
 	}
@@ -504,7 +736,7 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 	}
 	__syncthreads();
 
-	qrb_form_q<T, NW, NBK, RPL>(a, item, A, ld, Vb, Ts, tau, vv, N);
+	qrb_form_q<T, NW, NBK, GM>(a, item, A, ld, Vb, Ts, tau, vv, N);
 }
 
 // ----------------------------------------------- column-pivoted QR
@@ -806,7 +1038,7 @@ __global__ void __maxnreg__(96) k_qrp(QrArgs<T> a)
 	for (int p = w; p < np; p += NW)
 		qrb_block_t<T, NBK>(A, ld, tau, Ts + (size_t)p * NBK * NBK, N, p * NBK, min(NBK, N - p * NBK), lane);
 	__syncthreads();
-	qrb_form_q<T, NW, NBK, RPL>(a, item, A, ld, Vb, Ts, tau, vv, N);
+	qrb_form_q<T, NW, NBK, GM>(a, item, A, ld, Vb, Ts, tau, vv, N);
 }
 
 template <typename T>

@@ -87,10 +87,12 @@ __global__ void k_add_diag(int n, int NB, T *A, long long s)
 // block reflector I - V T^H V^H (larft forward, columnwise), 8 columns per warp
 // by DMMA (reflect8), so every trailing column is read twice and written once
 // per block.
-// Bound by latency: one CTA per item, M / 8 panels in series.  8x8, four sweeps
-// with unequal-time of one chain: 23.7 -> 23.0 ms; complex 10x10 x 64, with
-// k_qrb's complex panels through the same tiles: 98.6 -> 87.9 ms a sweep (k_qrb
-// 17 -> 12.2 ms of it), before: one column per warp.
+// Warps 0-3 take a panel's reflector to the next panel and factor that one
+// (qr_panel8) while the others take it to the remaining columns.  Bound by
+// latency: one CTA per item, M / 8 panels in series.  The class of one
+// unequal-time measurement, one column per warp at first: 8x8, one chain, 1.58 ms
+// with tiles alone, 0.77 ms with the register panels beside them; complex 10x10
+// x 64 16.6 -> 11.0 ms.
 
 template <typename T>
 struct HqrArgs {
@@ -102,142 +104,102 @@ struct HqrArgs {
 	unsigned *err;
 };
 
-template <typename T, int NBK, int NW>
+// warps of a panel and the look-ahead's; leading dimension of the reflectors
+// (4 mod 16: conflict-free tiles)
+constexpr int HQR_PW = 4;
+__host__ __device__ inline int hqr_ld(int M) { return (M + 11) / 16 * 16 + 4; }
+
+template <typename T, int NBK>
 size_t hqr_smem_bytes(int M)
 {
-	return sizeof(T) * ((size_t)M * NBK + NBK * NBK + NBK) + sizeof(double) * NW + 64;
+	return sizeof(T) * (2 * (size_t)hqr_ld(M) * NBK + 2 * NBK * NBK + NBK) + sizeof(double) * 2 * NBK;
 }
 
-template <typename T, int NBK, int NW>
+template <typename T, int NBK, int NW, int RP>
 __global__ void __launch_bounds__(NW * 32) k_hqr(HqrArgs<T> a)
 {
 	const int item = blockIdx.x;
 	if (item >= a.batch) return;
-	const int M = a.M, n = a.n, lda = a.lda;
+	const int M = a.M, n = a.n, ldv = hqr_ld(M);
+	const size_t lda = a.lda;
 	const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 	extern __shared__ __align__(16) unsigned char smraw[];
-	T *V = (T *)smraw;                    // rows j0.. of the panel, ld M
-	T *Tt = V + (size_t)M * NBK;          // NBK x NBK block-reflector factor
-	T *tau = Tt + NBK * NBK;
-	double *red = (double *)(tau + NBK);
+	T *Vb = (T *)smraw;                   // two panels from their first row on, ld ldv
+	T *Tb = Vb + 2 * (size_t)ldv * NBK;   // their NBK x NBK block-reflector factors
+	T *tau = Tb + 2 * NBK * NBK;
+	double *beta = (double *)(tau + NBK), *vv = beta + NBK;
+	__shared__ PanelShared<T, HQR_PW> sh;
 	T *A = a.A + a.aA.off(item);
 	T *Q = a.Qh + a.aQ.off(item);
 	T *X2 = a.nx2 ? a.X + a.aX.off(item) : nullptr;
-	if (n > M) {
+	if (n > M || M > 32 * HQR_PW * RP) {
 		if (tid == 0) atomicOr(a.err, DQ_ERR_SIZE);
 		return;
 	}
-	for (long long q = tid; q < (long long)M * M; q += NW * 32) {
-		const int r = (int)(q % M), c = (int)(q / M);
-		Q[q] = (r == c) ? one<T>() : zero<T>();
-	}
+	for (int q = tid; q < M * M; q += NW * 32) Q[q] = (q / M == q % M) ? one<T>() : zero<T>();
+	// panel p from Vb, where the look-ahead left it (p > 0), or from A: V stays in
+	// Vb, R goes to A with zeros below
 	bool bad = false;
+	auto panel = [&](int p) {
+		const int j0 = p * NBK, nb = min(NBK, n - j0);
+		T *Aj = A + j0 + lda * j0, *V = Vb + (size_t)(p & 1) * ldv * NBK;
+		qr_panel8<T, HQR_PW, RP>(
+			sh, M - j0, nb, w, lane, Tb + (p & 1) * NBK * NBK, tau, beta, vv,
+			[&](int r, int c) { return p ? V[r + (size_t)ldv * c] : Aj[r + lda * c]; },
+			[&](int r, int c, T v) {
+				V[r + (size_t)ldv * c] = v;
+				if (c < nb) Aj[r + lda * c] = (r <= c) ? v : zero<T>();
+			});
+		if (tid < nb && !(beta[tid] == beta[tid])) bad = true;
+	};
 	__syncthreads();
-	for (int j0 = 0; j0 < n; j0 += NBK) {
-		const int nb = min(NBK, n - j0);
-		const int mr = M - j0;
-		for (int q = tid; q < mr * nb; q += NW * 32) {
-			const int r = q % mr, c = q / mr;
-			V[r + (size_t)M * c] = A[(j0 + r) + (size_t)lda * (j0 + c)];
-		}
-		__syncthreads();
-		// unblocked QR of the panel (zgeqr2), reflectors stored below the diagonal
-		for (int k = 0; k < nb; k++) {
-			double s = 0.0;
-			for (int r = k + 1 + tid; r < mr; r += NW * 32) s += abs2(V[r + (size_t)M * k]);
-			s = warp_sum(s);
-			if (lane == 0) red[w] = s;
-			__syncthreads();
-			double sig = 0.0;
-			for (int q = 0; q < NW; q++) sig += red[q];
-			const T alpha = V[k + (size_t)M * k];
-			T tk, scal;
-			double beta;
-			if (sig == 0.0 && im(alpha) == 0.0) {
-				tk = zero<T>();
-				beta = re(alpha);
-				scal = zero<T>();
-			} else {
-				beta = -copysign(sqrt(abs2(alpha) + sig), re(alpha));
-				tk = (from_re<T>(beta) - alpha) / beta;
-				scal = one<T>() / (alpha - beta);
-			}
-			if (!(beta == beta)) bad = true;
-			__syncthreads();
-			for (int r = k + 1 + tid; r < mr; r += NW * 32) V[r + (size_t)M * k] *= scal;
-			if (tid == 0) {
-				V[k + (size_t)M * k] = from_re<T>(beta);
-				tau[k] = tk;
-			}
-			__syncthreads();
-			const T ct = conjv(tk);
-			for (int c = k + 1 + w; c < nb; c += NW) {
-				T dot = zero<T>();
-				for (int r = k + lane; r < mr; r += 32) {
-					const T v = (r == k) ? one<T>() : V[r + (size_t)M * k];
-					dot += conjv(v) * V[r + (size_t)M * c];
+	if (w < HQR_PW) panel(0);
+	__syncthreads();
+	const int np = (n + NBK - 1) / NBK;
+	for (int p = 0; p < np; p++) {
+		const int j0 = p * NBK, nb = min(NBK, n - j0), j1 = j0 + nb, mr = M - j0;
+		const T *V = Vb + (size_t)(p & 1) * ldv * NBK, *Tp = Tb + (p & 1) * NBK * NBK;
+		const bool next = j1 < n;
+		if (next && w < HQR_PW) {
+			// the next panel's columns and that panel
+			T *C = A + j0 + lda * j1, *Vn = Vb + (size_t)((p + 1) & 1) * ldv * NBK;
+			using ND = NextDepth<T, 4 * RP>;
+			reflect_next<T, HQR_PW, ND::AC, ND::RT>(
+				sh, min(NBK, n - j1), V, ldv, Tp, mr, nb, w, lane,
+				[&](int r, int c) { return C[r + lda * c]; },
+				[&](int r, int c, T v) {
+					if (r >= NBK) Vn[r - NBK + (size_t)ldv * c] = v;
+					else C[r + lda * c] = v;
+				});
+			bar_panel<HQR_PW>();
+			panel(p + 1);
+		} else {
+			// all other columns: of the panel and the nx1 right of it, X, Q
+			const int slot = next ? w - HQR_PW : w, ns = next ? NW - HQR_PW : NW;
+			const int c1 = min(j1 + NBK, n), n1 = n + a.nx1 - c1;
+			const int t1 = (n1 + 7) / 8, t2 = (a.nx2 + 7) / 8, t3 = (M + 7) / 8;
+			using D = ReflectDepth<T, true>;
+			for (int t = slot; t < t1 + t2 + t3; t += ns) {
+				T *C;
+				size_t ldc = lda;
+				int left;
+				if (t < t1) {
+					C = A + j0 + lda * (c1 + 8 * t);
+					left = n1 - 8 * t;
+				} else if (t < t1 + t2) {
+					C = X2 + j0 + lda * (8 * (t - t1));
+					left = a.nx2 - 8 * (t - t1);
+				} else {
+					ldc = M;
+					C = Q + j0 + ldc * (8 * (t - t1 - t2));
+					left = M - 8 * (t - t1 - t2);
 				}
-				dot = warp_sum(dot);
-				const T f = ct * dot;
-				for (int r = k + lane; r < mr; r += 32) {
-					const T v = (r == k) ? one<T>() : V[r + (size_t)M * k];
-					V[r + (size_t)M * c] -= v * f;
-				}
+				reflect8<T, true, D::AC, D::RT>(C, ldc, min(8, left), V, ldv, Tp, mr, nb, lane);
 			}
-			__syncthreads();
-		}
-		// R rows of the panel back to A, zeros below the diagonal
-		for (int q = tid; q < mr * nb; q += NW * 32) {
-			const int r = q % mr, c = q / mr;
-			A[(j0 + r) + (size_t)lda * (j0 + c)] = (r <= c) ? V[r + (size_t)M * c] : zero<T>();
-		}
-		// y[p][k] = v_p^H v_k (p < k), then T by the larft recurrence
-		for (int pk = w; pk < nb * nb; pk += NW) {
-			const int p = pk % nb, k = pk / nb;
-			if (p >= k) continue;
-			T dot = zero<T>();
-			for (int r = k + lane; r < mr; r += 32) {
-				const T vk = (r == k) ? one<T>() : V[r + (size_t)M * k];
-				dot += conjv(V[r + (size_t)M * p]) * vk;
-			}
-			dot = warp_sum(dot);
-			if (lane == 0) Tt[p + NBK * k] = dot;
-		}
-		__syncthreads();
-		if (tid == 0) {
-			for (int k = 0; k < nb; k++) {
-				T tmp[NBK];
-#pragma unroll
-				for (int p = 0; p < NBK; p++) {
-					T s = zero<T>();
-					if (p < k)
-						for (int q = p; q < k; q++) s += Tt[p + NBK * q] * Tt[q + NBK * k];
-					tmp[p] = -tau[k] * s;
-				}
-#pragma unroll
-				for (int p = 0; p < NBK; p++)
-					if (p < k) Tt[p + NBK * k] = tmp[p];
-				Tt[k + NBK * k] = tau[k];
-			}
-		}
-		__syncthreads();
-		// trailing columns: C -= V T^H (V^H C), rows j0..M-1, 8 columns a warp:
-		// those of the panel and the nx1 right of it, X, Q
-		const int n1 = n - j0 - nb + a.nx1, t1 = (n1 + 7) / 8, t2 = (a.nx2 + 7) / 8, t3 = (M + 7) / 8;
-		auto v = [&](int r, int k) {
-			return (k < nb && r >= k) ? ((r == k) ? one<T>() : V[r + (size_t)M * k]) : zero<T>();
-		};
-		for (int t = w; t < t1 + t2 + t3; t += NW) {
-			if (t < t1)
-				reflect8<T, true>(A + j0 + (size_t)lda * (j0 + nb), (size_t)lda, 8 * t, n1, v, Tt, 0, mr, nb, lane);
-			else if (t < t1 + t2)
-				reflect8<T, true>(X2 + j0, (size_t)lda, 8 * (t - t1), a.nx2, v, Tt, 0, mr, nb, lane);
-			else
-				reflect8<T, true>(Q + j0, (size_t)M, 8 * (t - t1 - t2), M, v, Tt, 0, mr, nb, lane);
 		}
 		__syncthreads();
 	}
-	if (bad && tid == 0) atomicOr(a.err, DQ_ERR_NAN);
+	if (bad) atomicOr(a.err, DQ_ERR_NAN);
 }
 
 // ------------------------------------------------ triangular block inverse

@@ -13,6 +13,9 @@ namespace dq {
 
 // 226 KB leaves room for the kernels' static shared memory
 static const size_t SMEM_FIT = 226 * 1024;
+// beside the panel's shared variables
+template <typename T>
+constexpr size_t qr_panel_fit() { return 227 * 1024 - sizeof(PanelShared<T, 4>) - 256; }
 
 // carve: the shared-memory forms take the largest shared-memory carveout
 // (room for a GEMM CTA beside them); the global-memory forms keep the
@@ -59,7 +62,7 @@ template <typename T>
 int launch_qr_presort(const QrArgs<T> &a, cudaStream_t st)
 {
 	if (a.N < 1 || a.N > max_dense_n<T>()) return DQMC_E_ARG;
-	if (qrb_smem_bytes<T, 8>(a.N) <= SMEM_FIT) return launch_qrb_gm<T, false>(a, st);
+	if (qrb_smem_bytes<T, 8>(a.N) <= qr_panel_fit<T>()) return launch_qrb_gm<T, false>(a, st);
 	if (!a.work) return DQMC_E_ARG;
 	return launch_qrb_gm<T, true>(a, st);
 }

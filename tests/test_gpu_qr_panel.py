@@ -45,3 +45,13 @@ def test_diagonal_factors(cplx, N):
     rc, G, _ = _call(C)
     assert rc == 0
     assert np.max(np.abs(G[0] - np.diag(1 / (1 + d[0].prod(0))))) < 1e-14
+
+
+@pytest.mark.parametrize("cplx,lo,hi", [(0, 140, 168), (1, 92, 124)])
+def test_every_size_where_the_matrix_leaves_one_sm(cplx, lo, hi):
+    pytest.importorskip("torch")
+    for N in range(lo, hi):
+        C = 0.8 * np.eye(N) + 0.3 * _random((1, 2, N, N), cplx, N) / np.sqrt(N)
+        rc, G, _ = _call(C)
+        assert rc == 0, N
+        assert np.max(np.abs(G[0] - np.linalg.inv(np.eye(N) + C[0, 1] @ C[0, 0]))) < 1e-10, N

@@ -576,32 +576,14 @@ __device__ inline void qrb_form_q(const QrArgs<T> &a, int item, T *A, int ld, T 
 	}
 }
 
-template <typename T, int NW, int NBK, int RPL, bool GM>
-__global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
+// pvt: the columns of X (rows when a.trans) in stable descending order of
+// their norms, scaled by dc (greens.c:123-129); the ranks in (int *)Vb when
+// a.trans.  vn: N doubles, Vb: 8 N elements of scratch.  All warps.
+template <typename T, int NW, int RPL>
+__device__ inline void qr_order(const QrArgs<T> &a, const T *X, const double *dc, int N, double *vn, int *pvt, T *Vb)
 {
-	const int item = blockIdx.x;
-	if (item >= a.batch) return;
-	const int N = a.N, ld = GM ? N : qrb_ld(N);
+	constexpr int NBK = 8;
 	const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-	const int np = (N + NBK - 1) / NBK;
-	extern __shared__ __align__(16) unsigned char smraw[];
-	// N columns, leading dimension ld, position order
-	T *A = GM ? a.work + (size_t)item * a.w_stride : (T *)smraw;
-	// copies of a panel's V (ld x NBK): one, in the global-memory form two
-	T *Vb = GM ? (T *)smraw : A + (size_t)ld * N;
-	T *tau = Vb + (GM ? 2 : 1) * (size_t)ld * NBK;   // N
-	T *Ts = tau + N;                            // np blocks of NBK x NBK
-	double *dsh = (double *)(Ts + (size_t)np * NBK * NBK);
-	double *vv = dsh + N;                       // v^H v
-	double *vn = vv + N;                        // squared column norms
-	int *pvt = (int *)(vn + N);
-	if (N > 32 * RPL) {
-		if (tid == 0 && a.err) atomicOr(a.err, DQ_ERR_SIZE);
-		return;
-	}
-	const T *X = a.X + (size_t)item * a.x_stride;
-	const double *dc = a.dcol ? a.dcol + (size_t)item * a.d_stride : nullptr;
-
 	if (a.trans) {
 		// norms of X's rows: a warp's lanes take 32 rows, a warp every NW-th column,
 		// the partial sums meet in Vb
@@ -654,6 +636,35 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 		if (a.trans) ((int *)Vb)[c] = rank;
 	}
 	__syncthreads();
+}
+
+template <typename T, int NW, int NBK, int RPL, bool GM>
+__global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
+{
+	const int item = blockIdx.x;
+	if (item >= a.batch) return;
+	const int N = a.N, ld = GM ? N : qrb_ld(N);
+	const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+	const int np = (N + NBK - 1) / NBK;
+	extern __shared__ __align__(16) unsigned char smraw[];
+	// N columns, leading dimension ld, position order
+	T *A = GM ? a.work + (size_t)item * a.w_stride : (T *)smraw;
+	// copies of a panel's V (ld x NBK): one, in the global-memory form two
+	T *Vb = GM ? (T *)smraw : A + (size_t)ld * N;
+	T *tau = Vb + (GM ? 2 : 1) * (size_t)ld * NBK;   // N
+	T *Ts = tau + N;                            // np blocks of NBK x NBK
+	double *dsh = (double *)(Ts + (size_t)np * NBK * NBK);
+	double *vv = dsh + N;                       // v^H v
+	double *vn = vv + N;                        // squared column norms
+	int *pvt = (int *)(vn + N);
+	if (N > 32 * RPL) {
+		if (tid == 0 && a.err) atomicOr(a.err, DQ_ERR_SIZE);
+		return;
+	}
+	const T *X = a.X + (size_t)item * a.x_stride;
+	const double *dc = a.dcol ? a.dcol + (size_t)item * a.d_stride : nullptr;
+
+	qr_order<T, NW, RPL>(a, X, dc, N, vn, pvt, Vb);
 	if (a.trans) {
 		const int *rk = (const int *)Vb;
 		for (int r = w; r < N; r += NW)
@@ -737,6 +748,207 @@ __global__ void __launch_bounds__(NW * 32) k_qrb(QrArgs<T> a)
 	__syncthreads();
 
 	qrb_form_q<T, NW, NBK, GM>(a, item, A, ld, Vb, Ts, tau, vv, N);
+}
+
+// ----------------------------------------------- the same over a cluster
+//
+// Few matrices that do not fit one SM's shared memory: the columns' 8-column
+// blocks lie round robin over the shared memory of a cluster of P CTAs (block b
+// in CTA b mod P).  A panel's owner factors it and writes its reflectors and T
+// to every CTA; each takes them to its own columns, the next panel's owner
+// with its first four warps on that panel; one cluster barrier per panel.  Q
+// backwards: each CTA copies the next block's reflectors from their owner
+// while the present block's are applied.
+// Bound by the panels' chain of latencies; with the matrix in L2 one SM's traffic
+// (64 bytes a cycle, three passes over the trailing columns per panel) is.  The
+// launcher's rule carries both sides' times.
+
+template <typename T>
+size_t qrc_smem_bytes(int N, int P)
+{
+	const int np = (N + 7) / 8, ld = qrb_ld(N), nl = (np + P - 1) / P;
+	return sizeof(T) * ((size_t)ld * 8 * nl + 2 * (size_t)ld * 8 + 2 * 64 + N) + sizeof(double) * 3 * (size_t)N
+	       + sizeof(int) * (size_t)N + 64;
+}
+
+// p of CTA `rank` of the cluster
+template <typename T>
+__device__ inline T *cluster_peer(T *p, int rank)
+{
+	unsigned long long r;
+	asm volatile("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"((unsigned long long)p), "r"(rank));
+	return (T *)r;
+}
+
+template <typename T, int NW, int RPL>
+__global__ void __launch_bounds__(NW * 32) k_qrc(QrArgs<T> a, int P)
+{
+	constexpr int NBK = 8;
+	const int item = blockIdx.x / P, rank = blockIdx.x % P;
+	const int N = a.N, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+	const size_t ld = qrb_ld(N);
+	const int np = (N + NBK - 1) / NBK, nl = (np + P - 1) / P;
+	extern __shared__ __align__(16) unsigned char smraw[];
+	T *A = (T *)smraw;                          // own blocks, 8 columns each
+	T *Vb = A + ld * NBK * nl;                  // two panels' reflectors from their first row on
+	T *Tb = Vb + 2 * ld * NBK;                  // their T
+	T *tau = Tb + 2 * NBK * NBK;                // N
+	double *dsh = (double *)(tau + N), *vv = dsh + N, *vn = vv + N;
+	int *pvt = (int *)(vn + N);
+	T *Tg = a.work + (size_t)item * a.w_stride; // every panel's T
+	const T *X = a.X + (size_t)item * a.x_stride;
+	const double *dc = a.dcol ? a.dcol + (size_t)item * a.d_stride : nullptr;
+	auto cluster_sync = []() {
+		asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+	};
+	// first own block >= b; local column of a global one
+	auto first = [&](int b) { return b <= rank ? 0 : (b - rank + P - 1) / P; };
+	auto block = [&](int b) { return A + ld * NBK * (b / P); };
+
+	qr_order<T, NW, RPL>(a, X, dc, N, vn, pvt, Vb);
+	if (a.trans) {
+		const int *rk = (const int *)Vb;
+		for (int c = lane; c < N; c += 32) {
+			const int j = rk[c], b = j / NBK;
+			if (b % P != rank) continue;
+			T *Aj = block(b) + ld * (j - b * NBK);
+			const double sc = dc ? dc[c] : 1.0;
+#pragma unroll 4
+			for (int r = w; r < N; r += NW) Aj[r] = conjv(X[c + (size_t)N * r]) * sc;
+		}
+	} else {
+#pragma unroll 2
+		for (int lc = w; lc < NBK * nl; lc += NW) {
+			const int j = (lc / NBK * P + rank) * NBK + lc % NBK;
+			if (j >= N) continue;
+			const int c = pvt[j];
+			const double sc = dc ? dc[c] : 1.0;
+			T e[RPL];
+#pragma unroll
+			for (int t = 0; t < RPL; t++) e[t] = lane + 32 * t < N ? X[lane + 32 * t + (size_t)N * c] : zero<T>();
+#pragma unroll
+			for (int t = 0; t < RPL; t++)
+				if (lane + 32 * t < N) A[lane + 32 * t + ld * lc] = e[t] * sc;
+		}
+	}
+	// also: every CTA of the cluster runs before the first remote write
+	cluster_sync();
+
+	using ND = NextDepth<T, RPL>;
+	using D = ReflectDepth<T, false>;
+	constexpr int PW = QrbPanel<T, RPL>::PW, RP = QrbPanel<T, RPL>::RP, GW = 4;
+	static_assert(PW <= GW && GW < NW, "panel warps among the look-ahead's");
+	__shared__ PanelShared<T, PW> sh;
+	auto panel = [&](int p) {
+		const int j0 = p * NBK, nb = min(NBK, N - j0);
+		T *Aj = block(p) + j0, *V = Vb + (p & 1) * ld * NBK, *Tp = Tb + (p & 1) * NBK * NBK;
+		qr_panel8<T, PW, RP>(
+			sh, N - j0, nb, w, lane, Tp, tau + j0, dsh + j0, vv + j0,
+			[&](int r, int c) { return Aj[r + ld * c]; },
+			[&](int r, int c, T v) {
+				if (c >= nb) return;
+				Aj[r + ld * c] = v;
+				for (int q = 0; q < P; q++) cluster_peer(V, q)[r + ld * c] = v;
+			});
+		if (w == PW - 1) {
+			__syncwarp();
+			for (int e = lane; e < NBK * NBK; e += 32) {
+				if (e % NBK > e / NBK || e / NBK >= nb) continue;
+				Tg[p * NBK * NBK + e] = Tp[e];
+				for (int q = 0; q < P; q++)
+					if (q != rank) cluster_peer(Tp, q)[e] = Tp[e];
+			}
+			if (lane < nb)
+				for (int q = 0; q < P; q++)
+					if (q != rank) {
+						cluster_peer(tau, q)[j0 + lane] = tau[j0 + lane];
+						cluster_peer(dsh, q)[j0 + lane] = dsh[j0 + lane];
+						cluster_peer(vv, q)[j0 + lane] = vv[j0 + lane];
+					}
+		}
+	};
+	if (rank == 0 && w < PW) panel(0);
+	cluster_sync();
+	for (int p = 0; p < np; p++) {
+		const int j0 = p * NBK, nb = min(NBK, N - j0), j1 = j0 + nb, mr = N - j0;
+		const T *V = Vb + (p & 1) * ld * NBK, *Tp = Tb + (p & 1) * NBK * NBK;
+		const bool next = j1 < N && (p + 1) % P == rank;
+		if (next && w < GW) {
+			T *C = block(p + 1) + j0;
+			reflect_next<T, GW, ND::AC, ND::RT>(
+				sh, min(NBK, N - j1), V, ld, Tp, mr, nb, w, lane,
+				[&](int r, int c) { return C[r + ld * c]; },
+				[&](int r, int c, T v) { C[r + ld * c] = v; });
+			bar_panel<GW>();
+			if (w < PW) panel(p + 1);
+		} else {
+			const int ns = next ? NW - GW : NW;
+			for (int l = first(p + 2) + (next ? w - GW : w); l * P + rank < np; l += ns)
+				reflect8<T, true, D::AC, D::RT>(A + j0 + ld * NBK * l, ld, min(NBK, N - NBK * (l * P + rank)), V,
+				                                ld, Tp, mr, nb, lane);
+		}
+		cluster_sync();
+	}
+
+	// D^-1 R in position order (Rs) or in the original one (Tout), diag(R)
+	// (0 -> 1) and the order
+	for (int lc = w; lc < NBK * nl; lc += NW) {
+		const int j = (lc / NBK * P + rank) * NBK + lc % NBK;
+		if (j >= N) continue;
+		T *out = a.Tout ? a.Tout + (size_t)item * a.t_stride + (size_t)N * pvt[j]
+		                : a.Rs + (size_t)item * a.r_stride + (size_t)N * j;
+		for (int r = lane; r < N; r += 32) {
+			const double dr = dsh[r] == 0.0 ? 1.0 : dsh[r];
+			out[r] = (r <= j) ? A[r + ld * lc] / dr : zero<T>();
+		}
+	}
+	if (rank == 0)
+		for (int r = tid; r < N; r += NW * 32) {
+			a.dout[(size_t)item * a.dout_stride + r] = dsh[r] == 0.0 ? 1.0 : dsh[r];
+			if (a.pvt) a.pvt[(size_t)item * a.p_stride + r] = pvt[r];
+		}
+
+	// Q = H_0 ... H_{N-1} backwards in place of A (qrb_form_q)
+	auto fetch = [&](int p) {
+		const int j0 = p * NBK, nb = min(NBK, N - j0);
+		const T *Aj = cluster_peer(block(p) + j0, p % P);
+		T *V = Vb + (p & 1) * ld * NBK;
+		for (int k = w & 7; k < nb; k += 8)
+#pragma unroll 4
+			for (int r = j0 + lane + 32 * (w >> 3); r < N; r += 64) V[r - j0 + ld * k] = Aj[r - j0 + ld * k];
+		if (tid < NBK * NBK) Tb[(p & 1) * NBK * NBK + tid] = Tg[p * NBK * NBK + tid];
+	};
+	fetch(np - 1);
+	cluster_sync();
+	for (int p = np - 1; p >= 0; p--) {
+		const int j0 = p * NBK, nb = min(NBK, N - j0), mr = N - j0;
+		if (p % P == rank) {
+			T *Aj = block(p) + j0;
+			for (int k = w; k < nb; k += NW)
+				for (int r = lane; r < mr; r += 32) Aj[r + ld * k] = (r == k) ? one<T>() : zero<T>();
+		}
+		for (int lc = NBK * first(p + 1) + w; lc < NBK * nl; lc += NW)
+			if (lane < nb) A[j0 + lane + ld * lc] = zero<T>();
+		if (p > 0) fetch(p - 1);
+		__syncthreads();
+		for (int l = first(p) + w; l * P + rank < np; l += NW)
+			reflect8<T, false, D::AC, D::RT>(A + j0 + ld * NBK * l, ld, min(NBK, N - NBK * (l * P + rank)),
+			                                 Vb + (p & 1) * ld * NBK, ld, Tb + (p & 1) * NBK * NBK, mr, nb, lane);
+		cluster_sync();
+	}
+	T *Q = a.Q + (size_t)item * a.q_stride;
+	for (int lc = w; lc < NBK * nl; lc += NW) {
+		const int j = (lc / NBK * P + rank) * NBK + lc % NBK;
+		if (j >= N) continue;
+		for (int r = lane; r < N; r += 32) Q[r + (size_t)N * j] = A[r + ld * lc];
+	}
+	if (rank == 0 && w == 0 && a.qdet) {
+		T ph = one<T>();
+		for (int j = lane; j < N; j += 32) ph = ph * phase_of(one<T>() - tau[j] * vv[j]);
+#pragma unroll
+		for (int o = 16; o > 0; o >>= 1) ph = ph * shfl_xor(ph, o);
+		if (lane == 0) a.qdet[item] = ph;
+	}
 }
 
 // ----------------------------------------------- column-pivoted QR

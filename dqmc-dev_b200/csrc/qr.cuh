@@ -11,6 +11,7 @@
 //         QR_PRESORT), blocked by 8 with DMMA block-reflector updates;
 //         both form Q explicitly (so that a later g*Q is a plain GEMM and
 //         diag(v) Q^H is elementwise), with the phase of det Q;
+// k_qrc   k_qrb's factorisation with the matrix over a cluster's shared memory;
 // k_recb  G = (D_b^-1 Q^H + D_s T)^-1 D_b^-1 Q^H (greens.c:157-178) by LU
 //         with partial row pivoting and two triangular solves, plus the
 //         phase of det G (greens.c:194-207); or the two-sided form of it for
@@ -269,7 +270,7 @@ __device__ inline void reflect_cols(T *A, size_t lda, int cfirst, int cend, cons
 // by that chain of latencies (about 1000 cycles a reflector, 300 of them the
 // square root and the division), so
 // - the columns rotate through the slots and the loop is not unrolled,
-// - the odd lanes divide by beta while the even ones divide by the pivot, and
+// - each lane forms one of the quotients 1 / (alpha - beta) and tau, and
 // - T is solved for at the end, one column a lane.
 // One column per warp with two barriers and two reductions per reflector before:
 // k_qrb 275 -> 201 us at N = 144 x 2, 1050 -> 800 us at N = 144 x 512, complex
@@ -278,7 +279,7 @@ __device__ inline void reflect_cols(T *A, size_t lda, int cfirst, int cend, cons
 // above the diagonal, V below, zero for c >= nb.
 template <typename T, int PW>
 struct PanelShared {
-	T red[2][PW][8], xrow[2][8], scal[PW][8], g[PW][8], y[8][8];
+	T red[2][PW][8], xrow[2][8], g[PW][8], y[8][8];
 	T wred[4][64];
 };
 
@@ -355,39 +356,48 @@ __device__ inline void qr_panel8(PanelShared<T, PW> &sh, int mr, int nb, int w, 
 			__syncwarp();
 			sig = re(shfl(sm, 0));
 		}
-		const T alpha = xr[0], xc = xr[cl], sy = sh.scal[w][(k + cl) & 7];
+		const T alpha = xr[0], xc = xr[cl];
 		const bool none = sig == 0.0 && im(alpha) == 0.0;
 		const double beta = none ? re(alpha) : -copysign(sqrt(abs2(alpha) + sig), re(alpha));
 		const T del = alpha - beta;
-		const double den = (lane & 1) ? beta : (is_cplx<T>::value ? abs2(del) : re(del));
-		const double iq = 1.0 / den, io = __shfl_xor_sync(0xffffffffu, iq, 1);
-		const double ib = (lane & 1) ? iq : io, ia = (lane & 1) ? io : iq;
-		T scal = is_cplx<T>::value ? conjv(del) * ia : from_re<T>(ia), tk = -(del * ib), sb = scal * ib;
-		if (none) scal = tk = sb = zero<T>();
-		// later columns: x_c -= u g, u = x_k with alpha - beta on the diagonal (v_k / scal)
-		const T g = (cl > 0 && cl < 8 - k) ? -((conjv(del) * xc + sm) * sb) : zero<T>();
+		// scal = 1 / del and tau = -del / beta, one quotient a lane
+		T tk, scal;
+		if constexpr (is_cplx<T>::value) {
+			const double q = ((lane & 1) ? im(del) : re(del)) / ((lane & 2) ? -beta : ((lane & 1) ? -abs2(del) : abs2(del)));
+			scal = T{__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1)};
+			tk = T{__shfl_sync(0xffffffffu, q, 2), __shfl_sync(0xffffffffu, q, 3)};
+		} else {
+			const double q = ((lane & 1) ? -del : 1.0) / ((lane & 1) ? beta : del);
+			const double o = shfl_xor(q, 1);
+			scal = (lane & 1) ? o : q;
+			tk = (lane & 1) ? q : o;
+		}
+		if (none) scal = tk = zero<T>();
+		// v_k^H x_c; later columns: x_c -= v_k g; earlier ones hold v_c already
+		const T dk = xc + conjv(scal) * sm;
+		const T g = (cl > 0 && cl < 8 - k) ? conjv(tk) * dk : zero<T>();
 		if ((lane & 3) == 0) sh.g[w][cl] = g;
 		__syncwarp();
-		if (r0 == k) x[0][0] = del;
+#pragma unroll
+		for (int t = 0; t < RP; t++)
+			if (t > 0 || r0 > k) x[0][t] *= scal;
 		T u[RP];
 #pragma unroll
-		for (int t = 0; t < RP; t++) u[t] = (t == 0 && r0 < k) ? zero<T>() : x[0][t];
+		for (int t = 0; t < RP; t++) u[t] = (t == 0 && r0 <= k) ? (r0 == k ? one<T>() : zero<T>()) : x[0][t];
+		if (r0 == k) x[0][0] = from_re<T>(beta);
 #pragma unroll
 		for (int s = 1; s < 8; s++) {
 			const T gs = sh.g[w][s];
 #pragma unroll
 			for (int t = 0; t < RP; t++) x[s][t] -= u[t] * gs;
 		}
-		if (lane == 0) sh.scal[w][k] = scal;
 		if (w == PW - 1) {
-			// earlier ones (unscaled in the registers): y = v_c^H v_k
 			if (lane == 0) {
 				tau[k] = tk;
 				beta_out[k] = beta;
 				vv[k] = 1.0 + sig * abs2(scal);
 			}
-			const T y = conjv(sy) * (scal * (conjv(xc) * del + conjv(sm)));
-			if (cl >= 8 - k && (lane & 3) == 0) sh.y[k + cl - 8][k] = y;
+			if (cl >= 8 - k && (lane & 3) == 0) sh.y[k + cl - 8][k] = conjv(dk);
 		}
 		rotate();
 	}
@@ -410,14 +420,10 @@ __device__ inline void qr_panel8(PanelShared<T, PW> &sh, int mr, int nb, int w, 
 	}
 #pragma unroll
 	for (int c = 0; c < 8; c++) {
-		const T sc = c < nb ? sh.scal[w][c] : zero<T>();
-		const double bc = c < nb ? beta_out[c] : 0.0;
 #pragma unroll
 		for (int t = 0; t < RP; t++) {
 			const int r = r0 + 32 * PW * t;
-			T v = x[c][t] * sc;
-			if (t == 0 && r0 <= c) v = (r0 < c) ? x[c][0] : from_re<T>(bc);
-			if (r < mr) store(r, c, v);
+			if (r < mr) store(r, c, x[c][t]);
 		}
 	}
 }

@@ -525,14 +525,22 @@ __device__ inline void flush_panels(T *G, size_t ldg, int N, int NC, int kc, con
 // half-warp fall in distinct banks
 __host__ __device__ inline int cl_ldg(int N) { return N + ((6 - N % 4) % 4); }
 
+// whether columns of a real G (N rows) can move 16 bytes at a time: every column
+// starts on 16 bytes.  G is the caller's in dqmc_gpu_update_delayed and need
+// only be aligned to its 8-byte numbers there.
+__host__ __device__ inline bool g_wide(const void *Gg, int N)
+{
+	return (N & 1) == 0 && ((uintptr_t)Gg & 15) == 0;
+}
+
 // nc columns of G (N rows) between device memory and shared memory (leading dimension
-// cl_ldg(N), even), by nwarp warps: 16 bytes at a time where N is even.  The
+// cl_ldg(N), even), by nwarp warps: 16 bytes at a time where g_wide allows.  The
 // load is asynchronous (cp.async): commit and wait follow.
 template <typename T>
 __device__ inline void g_load(T *Gs, const T *Gg, int N, int nc, int warp, int nwarp, int lane)
 {
 	const int ldg = cl_ldg(N);
-	const bool wide = (N & 1) == 0;
+	const bool wide = g_wide(Gg, N);
 	for (int col = warp; col < nc; col += nwarp) {
 		T *dst = Gs + (size_t)ldg * col;
 		const T *src = Gg + (size_t)N * col;
@@ -547,7 +555,7 @@ template <typename T>
 __device__ inline void g_store(T *Gg, const T *Gs, int N, int nc, int warp, int nwarp, int lane)
 {
 	const int ldg = cl_ldg(N);
-	const bool wide = (N & 1) == 0;
+	const bool wide = g_wide(Gg, N);
 	for (int col = warp; col < nc; col += nwarp) {
 		T *dst = Gg + (size_t)N * col;
 		const T *src = Gs + (size_t)ldg * col;

@@ -131,13 +131,15 @@ __device__ inline T qr_v8(const T *V, size_t ldv, int r, int k, int mr, int nb)
 // are read as they are, so columns k >= nb hold zeros there.  Fragment layouts
 // of m8n8k4: lane l holds A[l/4][l%4], B[l%4][l/4] and C[l/4][2(l%4) + {0,1}];
 // W moves from the C to the B layout by shuffles.  Absent columns are computed
-// on the last present one and not stored.  AC row quads and RT row tiles are in
-// flight at a time, more when C lies in global memory.
+// on the last present one and not stored.  W's row quads go round AC
+// accumulators, whose number alone sets the order of the sum; LD quads (a
+// multiple of AC) and RT row tiles are in flight at a time, more when C lies in
+// global memory.
 // Bound by the FP64 tensor pipe (16 cycles a DMMA and SM quarter) when all
 // warps have columns, else by the chain load - product - store; the full row
 // groups carry no row or column test, which cost more issue slots than the
 // products.
-template <typename T, bool HERM, int AC, int RT>
+template <typename T, bool HERM, int AC, int LD, int RT>
 __device__ inline void reflect8(T *C, size_t ldc, int ncol, const T *V, size_t ldv, const T *Tp, int mr,
 		int nb, int lane)
 {
@@ -157,17 +159,30 @@ __device__ inline void reflect8(T *C, size_t ldc, int ncol, const T *V, size_t l
 #pragma unroll
 		for (int u = 0; u < 2; u++) tile_mma(w[u % AC], av[u], bv[u]);
 	}
+	static_assert(LD % AC == 0, "whole rounds of the accumulators");
 	int r = 8;
 #pragma unroll 2
-	for (; r + 4 * AC <= mr; r += 4 * AC) {
-		T av[AC], bv[AC];
+	for (; r + 4 * LD <= mr; r += 4 * LD) {
+		T av[LD], bv[LD];
 #pragma unroll
-		for (int u = 0; u < AC; u++) {
+		for (int u = 0; u < LD; u++) {
 			av[u] = conjv(vb[r + 4 * u + lr]);
 			bv[u] = cb[r + 4 * u + lr];
 		}
 #pragma unroll
-		for (int u = 0; u < AC; u++) tile_mma(w[u], av[u], bv[u]);
+		for (int u = 0; u < LD; u++) tile_mma(w[u % AC], av[u], bv[u]);
+	}
+	if constexpr (LD > AC) {
+		for (; r + 4 * AC <= mr; r += 4 * AC) {
+			T av[AC], bv[AC];
+#pragma unroll
+			for (int u = 0; u < AC; u++) {
+				av[u] = conjv(vb[r + 4 * u + lr]);
+				bv[u] = cb[r + 4 * u + lr];
+			}
+#pragma unroll
+			for (int u = 0; u < AC; u++) tile_mma(w[u], av[u], bv[u]);
+		}
 	}
 	for (; r < mr; r += 4) {
 		const bool ok = r + lr < mr;
@@ -232,10 +247,13 @@ __device__ inline void reflect8(T *C, size_t ldc, int ncol, const T *V, size_t l
 	for (; r < mr; r += 8) edge(r, false);
 }
 
-// depths of reflect8 for columns in shared and in global memory
+// depths of reflect8 for columns in shared and in global memory: the same
+// accumulators in both, so that a QR gives the same bits wherever its matrix
+// lies (the form goes by the items of a launch, which a lane count changes)
 template <typename T, bool GMEM>
 struct ReflectDepth {
-	static constexpr int AC = is_cplx<T>::value ? (GMEM ? 4 : 2) : (GMEM ? 8 : 4);
+	static constexpr int AC = is_cplx<T>::value ? 2 : 4;
+	static constexpr int LD = GMEM ? 2 * AC : AC;
 	static constexpr int RT = is_cplx<T>::value ? (GMEM ? 4 : 2) : (GMEM ? 8 : 3);
 };
 
@@ -254,7 +272,7 @@ __device__ inline void reflect_cols(T *A, size_t lda, int cfirst, int cend, cons
 {
 	using D = ReflectDepth<T, GMEM>;
 	for (int c = cfirst + 8 * slot; c < cend; c += 8 * nslots)
-		reflect8<T, HERM, D::AC, D::RT>(A + lda * c, lda, min(8, cend - c), Vp, ldv, Tp, mr, nb, lane);
+		reflect8<T, HERM, D::AC, D::LD, D::RT>(A + lda * c, lda, min(8, cend - c), Vp, ldv, Tp, mr, nb, lane);
 }
 
 // ----------------------------------------------- panel of 8 columns
@@ -890,7 +908,7 @@ __global__ void __launch_bounds__(NW * 32) k_qrc(QrArgs<T> a, int P)
 		} else {
 			const int ns = next ? NW - GW : NW;
 			for (int l = first(p + 2) + (next ? w - GW : w); l * P + rank < np; l += ns)
-				reflect8<T, true, D::AC, D::RT>(A + j0 + ld * NBK * l, ld, min(NBK, N - NBK * (l * P + rank)), V,
+				reflect8<T, true, D::AC, D::LD, D::RT>(A + j0 + ld * NBK * l, ld, min(NBK, N - NBK * (l * P + rank)), V,
 				                                ld, Tp, mr, nb, lane);
 		}
 		cluster_sync();
@@ -938,7 +956,7 @@ __global__ void __launch_bounds__(NW * 32) k_qrc(QrArgs<T> a, int P)
 		if (p > 0) fetch(p - 1);
 		__syncthreads();
 		for (int l = first(p) + w; l * P + rank < np; l += NW)
-			reflect8<T, false, D::AC, D::RT>(A + j0 + ld * NBK * l, ld, min(NBK, N - NBK * (l * P + rank)),
+			reflect8<T, false, D::AC, D::LD, D::RT>(A + j0 + ld * NBK * l, ld, min(NBK, N - NBK * (l * P + rank)),
 			                                 Vb + (p & 1) * ld * NBK, ld, Tb + (p & 1) * NBK * NBK, mr, nb, lane);
 		cluster_sync();
 	}

@@ -657,25 +657,29 @@ static cudaError_t update_attr(int N, int kd, int ldp, int split)
 template <typename T>
 static int launch_update(const UpdArgs<T> &a, cudaStream_t st, int split)
 {
+	cudaLaunchConfig_t cfg = {};
+	cudaLaunchAttribute at = {};
+	cfg.stream = st;
+	cudaError_t e;
 	if (split) {
-		cudaLaunchConfig_t cfg = {};
-		cudaLaunchAttribute at = {};
 		at.id = cudaLaunchAttributeClusterDimension;
 		at.val.clusterDim.x = 2 * split;
 		at.val.clusterDim.y = at.val.clusterDim.z = 1;
 		cfg.gridDim = dim3(2 * split * a.nchain);
 		cfg.blockDim = dim3(cl_warps(a.N) * 32 + 32);
 		cfg.dynamicSmemBytes = update_cl_smem_bytes<T>(a.N, split, a.n_delay);
-		cfg.stream = st;
 		cfg.attrs = &at;
 		cfg.numAttrs = 1;
-		return cudaLaunchKernelEx(&cfg, k_update_cl<T>, a) == cudaSuccess ? 0 : DQMC_E_CUDA;
+		e = cudaLaunchKernelEx(&cfg, k_update_cl<T>, a);
+	} else {
+		cfg.gridDim = dim3(a.nchain);
+		cfg.blockDim = dim3(update_warps(a.N) * 32 + 32);
+		cfg.dynamicSmemBytes = update_smem_bytes<T>(a.N, a.n_delay, a.ldp);
+		e = cudaLaunchKernelEx(&cfg, cfg.blockDim.x <= 352 ? k_update<T> : k_update_big<T>, a);
 	}
-	const int threads = update_warps(a.N) * 32 + 32;
-	const size_t smem = update_smem_bytes<T>(a.N, a.n_delay, a.ldp);
-	if (threads <= 352) k_update<T><<<a.nchain, threads, smem, st>>>(a);
-	else k_update_big<T><<<a.nchain, threads, smem, st>>>(a);
-	return 0;
+	if (e == cudaSuccess) return 0;
+	fprintf(stderr, "dqmc_b200: update launch failed: %s\n", cudaGetErrorString(e));
+	return DQMC_E_CUDA;
 }
 
 struct GroupBase {
@@ -1429,7 +1433,7 @@ struct Group : GroupBase, ProfHook {
 		launch_count++;
 	}
 
-	void update(int l)
+	int update(int l)
 	{
 		UpdArgs<T> a;
 		a.N = N; a.L = L; a.n_delay = kd; a.nchain = C; a.slice = l; a.ldp = ldp;
@@ -1440,11 +1444,12 @@ struct Group : GroupBase, ProfHook {
 		// slice again (L = 1), whose fields this kernel is still changing
 		a.next_slice = (L == 1) ? -1 : (l + 1) % L;
 		prof_begin(1);
-		launch_update<T>(a, st, upd_split);
+		if (const int rc = launch_update<T>(a, st, upd_split)) return rc;
 		prof_end(PC_UPDATE, 0.0, 0.0);
 		launch_count++;
 		watchdog("k_update");
 		if (L == 1) draws(0);
+		return 0;
 	}
 
 	// G <- B_l G B_l^-1 = exp_K (D G D^-1) inv_exp_K
@@ -1790,7 +1795,7 @@ struct Group : GroupBase, ProfHook {
 			if (rc) return rc;
 		}
 		for (int l = 0; l < L; l++) {
-			update(l);
+			if (const int rc = update(l)) return rc;
 			const int f = l / nmul;
 			const bool recalc = ((l + 1) % nmul) == 0;
 			if (recalc) {
@@ -3109,9 +3114,10 @@ static int seam_update(int batch, int N, int n_delay, const double *del, uint64_
 	a.N = N; a.L = 1; a.n_delay = kd; a.nchain = batch; a.slice = 0; a.ldp = ldp;
 	a.del = del; a.rng = rng; a.rng_ckpt = ck; a.hs = hs; a.G = (T *)G; a.phase = (T *)phase;
 	a.order = ord; a.u = uu; a.next_slice = -1;
-	launch_update<T>(a, st, split);
-	CK(cudaGetLastError());
+	const int rc = launch_update<T>(a, st, split);
 	CK(cudaStreamSynchronize(st));
+	if (rc) return rc;
+	CK(cudaGetLastError());
 	return 0;
 }
 

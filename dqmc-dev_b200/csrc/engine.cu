@@ -3106,19 +3106,24 @@ static int seam_update(int batch, int N, int n_delay, const double *del, uint64_
 	uint64_t *ck;
 	int *ord;
 	double *uu;
+	unsigned *err;
 	sc.add(ck, (size_t)batch * 17); sc.add(ord, (size_t)batch * 2 * N); sc.add(uu, (size_t)batch * 2 * N);
+	sc.add(err, 1);
 	if (sc.commit()) return DQMC_E_NOMEM;
+	CK(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
 	k_draws<<<batch, 32, draws_smem_bytes(N), st>>>(N, 1, batch, 0, del, rng, ck, hs, ord, uu);
 	UpdArgs<T> a;
 	memset(&a, 0, sizeof(a));
 	a.N = N; a.L = 1; a.n_delay = kd; a.nchain = batch; a.slice = 0; a.ldp = ldp;
 	a.del = del; a.rng = rng; a.rng_ckpt = ck; a.hs = hs; a.G = (T *)G; a.phase = (T *)phase;
-	a.order = ord; a.u = uu; a.next_slice = -1;
+	a.order = ord; a.u = uu; a.next_slice = -1; a.err = err;
 	const int rc = launch_update<T>(a, st, split);
+	unsigned e = 0;
+	CK(cudaMemcpyAsync(&e, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));
 	if (rc) return rc;
 	CK(cudaGetLastError());
-	return 0;
+	return e ? DQMC_E_DEVICE : 0;
 }
 
 template <typename T>

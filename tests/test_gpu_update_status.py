@@ -1,9 +1,10 @@
 """Status of the delayed update: a launch that the runtime refuses ends the call
-with an error instead of a sweep without its update.
+with an error instead of a sweep without its update, and an error word that the
+kernel has set (a wait that ran out) reaches the seam's caller.
 
-The refusal comes from a fake: the library's objects are linked once more with
-the runtime's launch call wrapped, and the wrapper returns an error code without
-launching when it is told to.
+Both come from a fake: the library's objects are linked once more with two calls
+of the runtime wrapped, and when they are told to, the launch returns an error
+code without launching and the copy of an error word to the host brings one.
 """
 import ctypes as C
 import glob
@@ -20,7 +21,7 @@ pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 PKG = os.path.join(ROOT, "dqmc-dev_b200")
-DQMC_E_CUDA = -11
+DQMC_E_CUDA, DQMC_E_DEVICE = -11, -13
 
 FAKE = r"""
 #include <cuda_runtime.h>
@@ -34,6 +35,17 @@ cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *
 		return cudaErrorLaunchOutOfResources;
 	}
 	return __real_cudaLaunchKernelExC(c, f, a);
+}
+unsigned fake_word = 0;   /* the error word the next 4-byte copy to the host brings */
+cudaError_t __real_cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t st);
+cudaError_t __wrap_cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t st)
+{
+	if (fake_word && n == sizeof(unsigned) && k == cudaMemcpyDeviceToHost) {
+		*(unsigned *)d = fake_word;
+		fake_word = 0;
+		return cudaSuccess;
+	}
+	return __real_cudaMemcpyAsync(d, s, n, k, st);
 }
 }
 """
@@ -51,7 +63,7 @@ def fake(tmp_path_factory):
     (d / "fake.cu").write_text(FAKE)
     so = str(d / "libfake.so")
     subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-cudart", "static",
-                    "-Xcompiler", "-fPIC", "-Xlinker", "--wrap=cudaLaunchKernelExC", "-o", so,
+                    "-Xcompiler", "-fPIC", "-Xlinker", "--wrap=cudaLaunchKernelExC", "-Xlinker", "--wrap=cudaMemcpyAsync", "-o", so,
                     str(d / "fake.cu")] + objs, check=True)
     from dqmc_b200 import lib
     own, lib._lib = lib._lib, None
@@ -113,3 +125,14 @@ def test_sweep_reports_a_refused_update(fake, form, monkeypatch):
         e.close()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("form", ["global", "cluster"])
+def test_seam_reports_the_kernels_error_word(fake, form, monkeypatch):
+    h, _ = fake
+    word = C.c_uint.in_dll(h, "fake_word")
+    word.value = 4
+    rc, _, _ = _seam(h, 32, form, monkeypatch)
+    assert word.value == 0 and rc == DQMC_E_DEVICE
+    rc, _, _ = _seam(h, 32, form, monkeypatch)
+    assert rc == 0

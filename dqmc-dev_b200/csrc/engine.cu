@@ -357,6 +357,7 @@ struct Slab {
 	{
 		if (cudaMalloc(&base, size ? size : 256) != cudaSuccess) {
 			base = nullptr;
+			cudaGetLastError();   // answered here: a later call must not see it
 			return DQMC_E_NOMEM;
 		}
 		for (auto &i : items) {
@@ -390,6 +391,7 @@ struct DevBuf {
 		if (count == 0) return 0;
 		if (cudaMalloc(&p, sizeof(T) * count) != cudaSuccess) {
 			p = nullptr;
+			cudaGetLastError();
 			return DQMC_E_NOMEM;
 		}
 		cudaMemset(p, 0, sizeof(T) * count);
@@ -692,6 +694,9 @@ struct GroupBase {
 	                       const int *hs, int sweep) = 0;
 	virtual int get_chains(int c0, int n, uint64_t *rng, int *hs, int *sweep, int *eqn, void *eq,
 	                       int *uen, void *ue) = 0;
+	// memory of the sweep's stack, and without it again
+	virtual int take_stack() { return 0; }
+	virtual void drop_stack() {}
 	virtual int init() = 0;
 	// init without waiting for it on the host
 	virtual int init_async() = 0;
@@ -820,8 +825,11 @@ struct Group : GroupBase, ProfHook {
 	} ok;
 	// The stack of a sweep: for f = 1 .. F-1 the decomposition of the clusters
 	// still to come, C_{F-1} ... C_f = T_f^H D_f Q_f^H, per f and item (f - 1
-	// first), built at the sweep's start from the last sweep's clusters
-	DevBuf<T> QL, TL, qdL;
+	// first), built at the sweep's start from the last sweep's clusters.  Q_f
+	// takes the place of C_f in Cl, which is spent there and formed anew before
+	// the stack's entry is: during a sweep the slots past the present cluster
+	// hold Q_f, between sweeps all of them hold clusters.
+	DevBuf<T> TL, qdL;
 	DevBuf<double> dL;
 	bool stack = false;
 	Slab slab, stack_slab;             // the buffers of create(), and the stack's
@@ -853,7 +861,7 @@ struct Group : GroupBase, ProfHook {
 		for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
 		if (jev) cudaEventDestroy(jev);
 		DevBuf<T> *tb[] = {&expK, &iexpK, &ehK, &iehK, &peu, &ped, &phase, &G, &Cl, &Qm, &Tm,
-		                   &Tm2, &Rs, &X, &W, &Gh, &acc_eq, &acc_ue, &phi, &qdet, &Sg, &QL, &TL, &qdL,
+		                   &Tm2, &Rs, &X, &W, &Gh, &acc_eq, &acc_ue, &phi, &qdet, &Sg, &TL, &qdL,
 		                   &ppu, &ppd, &ppru, &pprd, &gs_eq, &gs_ue};
 		for (auto *b : tb) b->release();
 		DevBuf<int> *ib[] = {&i_off, &i_idx, &ij_off, &ij_idx, &bb_off, &bb_idx, &bonds, &hs,
@@ -991,12 +999,6 @@ struct Group : GroupBase, ProfHook {
 		if (slab.commit()) return DQMC_E_NOMEM;
 		cudaMemset(slab.base, 0, slab.size);
 		if (p.period_uneqlt > 0 && ue.alloc(N, L, F, NB)) return DQMC_E_NOMEM;
-		// without room for the stack every recalculation takes the whole chain
-		const size_t ns = (size_t)std::max(F - 1, 0) * NB;
-		QL.take(stack_slab, ns * NN); TL.take(stack_slab, ns * NN);
-		qdL.take(stack_slab, ns); dL.take(stack_slab, ns * N);
-		stack = !stack_slab.commit();
-		if (!stack) cudaGetLastError();
 		// parameter matrices, per spin
 		auto up2 = [&](DevBuf<T> &dst, const void *u, const void *d) {
 			cudaMemcpy(dst.p, u, sizeof(T) * NN, cudaMemcpyHostToDevice);
@@ -1039,6 +1041,22 @@ struct Group : GroupBase, ProfHook {
 		CK(update_attr<T>(N, kd, ldp, upd_split));
 		CK(cudaDeviceSynchronize());
 		return 0;
+	}
+
+	// the stack's memory, once every lane has its other buffers
+	int take_stack() override
+	{
+		const size_t NN = (size_t)N * N, ns = (size_t)(F - 1) * NB;
+		TL.take(stack_slab, ns * NN);
+		qdL.take(stack_slab, ns); dL.take(stack_slab, ns * N);
+		stack = !stack_slab.commit();
+		return stack ? 0 : DQMC_E_NOMEM;
+	}
+	void drop_stack() override
+	{
+		stack = false;
+		stack_slab.release();
+		TL.release(); qdL.release(); dL.release();
 	}
 
 	int set_chain(int c, const double *e, const double *d, const uint64_t *r, const int *h,
@@ -1318,8 +1336,8 @@ struct Group : GroupBase, ProfHook {
 	// its order from the initial norms as all later ones leaves the error of G
 	// as it was and the launch of k_qrb in place of k_qrp (us, two items:
 	// N = 144 270 for 680, N = 256 1480 for 4440)
-	int qdt(const T *Xin, long long xs, bool trans, const double *dprev, const T *Tprev, T *Q, double *d,
-	        T *Tout, T *qd)
+	int qdt(const T *Xin, long long xs, bool trans, const double *dprev, const T *Tprev, T *Q, long long qs,
+	        double *d, T *Tout, T *qd)
 	{
 		const long long NN = (long long)N * N;
 		const double qfl = dense_flops<T>(N, NB), qby = 3.0 * sizeof(T) * NN * NB;
@@ -1327,7 +1345,7 @@ struct Group : GroupBase, ProfHook {
 		memset(&q, 0, sizeof(q));
 		q.N = N; q.batch = NB; q.err = err.p;
 		q.X = Xin; q.x_stride = xs; q.trans = trans;
-		q.Q = Q; q.q_stride = NN;
+		q.Q = Q; q.q_stride = qs;
 		q.dout = d; q.dout_stride = N;
 		q.qdet = qd;
 		q.pvt = pvt.p; q.p_stride = N;
@@ -1352,22 +1370,21 @@ struct Group : GroupBase, ProfHook {
 		return 0;
 	}
 
-	// the decompositions of C_{F-1} ... C_f for f = F-1 .. 1
+	// the decompositions of C_{F-1} ... C_f for f = F-1 .. 1, Q_f over C_f
+	// (qdt's kernels read their whole input before they write Q)
 	int build_stack()
 	{
-		const long long NN = (long long)N * N;
-		const Addr aC = per_item((long long)F * NN), aI = per_item(NN);
+		const long long NN = (long long)N * N, FNN = (long long)F * NN;
+		const Addr aC = per_item(FNN), aI = per_item(NN);
 		for (int f = F - 1; f >= 1; f--) {
 			const size_t o = (size_t)(f - 1) * NB, op = (size_t)f * NB;
-			const T *Cf = Cl.p + (size_t)f * NN;
+			T *Cf = Cl.p + (size_t)f * NN;
 			int rc;
 			if (f == F - 1) {
-				rc = qdt(Cf, (long long)F * NN, true, nullptr, nullptr, QL.p + o * NN, dL.p + o * N, TL.p + o * NN,
-				         qdL.p + o);
+				rc = qdt(Cf, FNN, true, nullptr, nullptr, Cf, FNN, dL.p + o * N, TL.p + o * NN, qdL.p + o);
 			} else {
-				gemm(gargs<T>(N, N, N, NB, Cf, aC, N, QL.p + op * NN, aI, N, X.p, aI, N, one<T>(), zero<T>(), GM_A_CT));
-				rc = qdt(X.p, NN, false, dL.p + op * N, TL.p + op * NN, QL.p + o * NN, dL.p + o * N, TL.p + o * NN,
-				         qdL.p + o);
+				gemm(gargs<T>(N, N, N, NB, Cf, aC, N, Cf + NN, aC, N, X.p, aI, N, one<T>(), zero<T>(), GM_A_CT));
+				rc = qdt(X.p, NN, false, dL.p + op * N, TL.p + op * NN, Cf, FNN, dL.p + o * N, TL.p + o * NN, qdL.p + o);
 			}
 			if (rc) return rc;
 		}
@@ -1386,14 +1403,15 @@ struct Group : GroupBase, ProfHook {
 		const T *Cf = Cl.p + (size_t)f * NN;
 		int rc;
 		if (f == 0) {
-			rc = qdt(Cf, (long long)F * NN, false, nullptr, nullptr, Qm.p, dR.p, Tn, qdet.p);
+			rc = qdt(Cf, (long long)F * NN, false, nullptr, nullptr, Qm.p, NN, dR.p, Tn, qdet.p);
 		} else {
 			gemm(gargs<T>(N, N, N, NB, Cf, aC, N, Qm.p, aI, N, X.p, aI, N));
-			rc = qdt(X.p, NN, false, dR.p, To, Qm.p, dR.p, Tn, qdet.p);
+			rc = qdt(X.p, NN, false, dR.p, To, Qm.p, NN, dR.p, Tn, qdet.p);
 		}
 		if (rc) return rc;
 		const bool two = f + 1 < F;
 		const size_t o = (size_t)f * NB;       // f + 1 in the stack
+		const T *Qf = Cf + NN;
 		RecArgs<T> ra;
 		memset(&ra, 0, sizeof(ra));
 		ra.N = N; ra.batch = NB;
@@ -1406,7 +1424,7 @@ struct Group : GroupBase, ProfHook {
 		ra.Tm = Tn; ra.t_stride = NN;
 		ra.G = G.p; ra.g_stride = NN;
 		if (two) {
-			gemm(gargs<T>(N, N, N, NB, Qm.p, aI, N, QL.p + o * NN, aI, N, X.p, aI, N, one<T>(), zero<T>(), GM_A_CT));
+			gemm(gargs<T>(N, N, N, NB, Qm.p, aI, N, Qf, aC, N, X.p, aI, N, one<T>(), zero<T>(), GM_A_CT));
 			gemm(gargs<T>(N, N, N, NB, Tn, aI, N, TL.p + o * NN, aI, N, Rs.p, aI, N, one<T>(), zero<T>(), GM_B_CT));
 			ra.Wl = X.p; ra.wl_stride = NN;
 			ra.Tm = Rs.p;
@@ -1420,7 +1438,7 @@ struct Group : GroupBase, ProfHook {
 		if (launch_rec<T>(ra, st)) return DQMC_E_ARG;
 		prof_end(PC_RECOMBINE, dense_flops<T>(N, NB), 3.0 * sizeof(T) * NN * NB);
 		launch_count++;
-		if (two) gemm(gargs<T>(N, N, N, NB, QL.p + o * NN, aI, N, To, aI, N, G.p, aI, N));
+		if (two) gemm(gargs<T>(N, N, N, NB, Qf, aC, N, To, aI, N, G.p, aI, N));
 		watchdog("recalc_g");
 		return combine_phase();
 	}
@@ -1893,7 +1911,10 @@ struct Group : GroupBase, ProfHook {
 			const int kind = (meq ? 1 : 0) | (mue ? 2 : 0);
 			if (debug_sync) {
 				int rc = enqueue_sweep(meq, mue);
-				if (rc) return rc;
+				if (rc) {
+					need_init = true;   // the clusters may be half replaced
+					return rc;
+				}
 				sweep++;
 				continue;
 			}
@@ -1950,7 +1971,10 @@ struct Group : GroupBase, ProfHook {
 		precs.clear();
 		int rc = enqueue_sweep(meq, mue);
 		profiling = false;
-		if (rc) return rc;
+		if (rc) {
+			need_init = true;
+			return rc;
+		}
 		CK(cudaMemcpyAsync(acc1.data(), nacc.p, sizeof(int) * C, cudaMemcpyDeviceToHost, st));
 		CK(cudaStreamSynchronize(st));
 		sweep++;
@@ -2035,14 +2059,22 @@ struct Group : GroupBase, ProfHook {
 		CK(cudaMemsetAsync(Sg.p, 0, sizeof(T) * NB * NN, st));
 		if (stack) {
 			const int rc = build_stack();
-			if (rc) return rc;
+			if (rc) {
+				need_init = true;
+				return rc;
+			}
 		}
 		for (int l = 0; l < L; l++) {
 			k_grad_acc<T><<<grid_for((long long)NB * NN), 256, 0, st>>>(N, NB, L, l, G.p, dv.p, dvi.p, Sg.p);
 			launch_count++;
 			if ((l + 1) % nmul == 0) {
+				// the stack's Q lies where the cluster was
+				if (stack) build_cluster(l / nmul);
 				const int rc = recalc_g(l / nmul);
-				if (rc) return rc;
+				if (rc) {
+					need_init = true;
+					return rc;
+				}
 			} else {
 				wrap(l);
 			}
@@ -2440,6 +2472,15 @@ struct Lanes : GroupBase {
 			g.push_back(x);
 			c0.push_back(c0.back() + n);
 		}
+		// All lanes sweep with a stack or none: the two ways round differently.
+		// With it an item has 2 F + 7 matrices.
+		for (GroupBase *x : g)
+			if (x->take_stack()) {
+				for (GroupBase *y : g) y->drop_stack();
+				fprintf(stderr, "dqmc_b200: no device memory for the sweep's stack, every recalculation of G "
+				        "takes the whole chain of clusters\n");
+				break;
+			}
 		return 0;
 	}
 

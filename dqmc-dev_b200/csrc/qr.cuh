@@ -132,9 +132,8 @@ __device__ inline T qr_v8(const T *V, size_t ldv, int r, int k, int mr, int nb)
 // of m8n8k4: lane l holds A[l/4][l%4], B[l%4][l/4] and C[l/4][2(l%4) + {0,1}];
 // W moves from the C to the B layout by shuffles.  Absent columns are computed
 // on the last present one and not stored.  W's row quads go round AC
-// accumulators, whose number alone sets the order of the sum; LD quads (a
-// multiple of AC) and RT row tiles are in flight at a time, more when C lies in
-// global memory.
+// accumulators, whose number alone sets the order of the sum; LD quads and RT row
+// tiles are in flight at a time, more when C lies in global memory.
 // Bound by the FP64 tensor pipe (16 cycles a DMMA and SM quarter) when all
 // warps have columns, else by the chain load - product - store; the full row
 // groups carry no row or column test, which cost more issue slots than the
@@ -159,34 +158,29 @@ __device__ inline void reflect8(T *C, size_t ldc, int ncol, const T *V, size_t l
 #pragma unroll
 		for (int u = 0; u < 2; u++) tile_mma(w[u % AC], av[u], bv[u]);
 	}
-	static_assert(LD % AC == 0, "whole rounds of the accumulators");
+	// quad q to accumulator q % AC, loads LD at a time
+	constexpr int B = AC > LD ? AC : LD;
+	static_assert(B % AC == 0 && B % LD == 0, "whole rounds");
 	int r = 8;
 #pragma unroll 2
-	for (; r + 4 * LD <= mr; r += 4 * LD) {
-		T av[LD], bv[LD];
+	for (; r + 4 * B <= mr; r += 4 * B) {
 #pragma unroll
-		for (int u = 0; u < LD; u++) {
-			av[u] = conjv(vb[r + 4 * u + lr]);
-			bv[u] = cb[r + 4 * u + lr];
-		}
+		for (int g = 0; g < B; g += LD) {
+			T av[LD], bv[LD];
 #pragma unroll
-		for (int u = 0; u < LD; u++) tile_mma(w[u % AC], av[u], bv[u]);
-	}
-	if constexpr (LD > AC) {
-		for (; r + 4 * AC <= mr; r += 4 * AC) {
-			T av[AC], bv[AC];
-#pragma unroll
-			for (int u = 0; u < AC; u++) {
-				av[u] = conjv(vb[r + 4 * u + lr]);
-				bv[u] = cb[r + 4 * u + lr];
+			for (int u = 0; u < LD; u++) {
+				av[u] = conjv(vb[r + 4 * (g + u) + lr]);
+				bv[u] = cb[r + 4 * (g + u) + lr];
 			}
 #pragma unroll
-			for (int u = 0; u < AC; u++) tile_mma(w[u], av[u], bv[u]);
+			for (int u = 0; u < LD; u++) tile_mma(w[(g + u) % AC], av[u], bv[u]);
 		}
 	}
-	for (; r < mr; r += 4) {
-		const bool ok = r + lr < mr;
-		tile_mma(w[0], ok ? conjv(vb[r + lr]) : zero<T>(), ok ? cb[r + lr] : zero<T>());
+#pragma unroll
+	for (int u = 0; u < B; u++) {
+		if (r + 4 * u >= mr) break;
+		const bool ok = r + 4 * u + lr < mr;
+		tile_mma(w[u % AC], ok ? conjv(vb[r + 4 * u + lr]) : zero<T>(), ok ? cb[r + 4 * u + lr] : zero<T>());
 	}
 #pragma unroll
 	for (int u = AC / 2; u > 0; u /= 2)
@@ -249,11 +243,15 @@ __device__ inline void reflect8(T *C, size_t ldc, int ncol, const T *V, size_t l
 
 // depths of reflect8 for columns in shared and in global memory: the same
 // accumulators in both, so that a QR gives the same bits wherever its matrix
-// lies (the form goes by the items of a launch, which a lane count changes)
+// lies (the form goes by the items of a launch, which a lane count changes).
+// Eight for complex scalars, whose terms are two products each: with two, G of
+// complex Hubbard clusters was 12 to 18% further from the exact one (N = 64 to
+// 144) than with the shuffled sums that the tiles replaced, with eight 4 to 5%, at
+// the same time a launch.
 template <typename T, bool GMEM>
 struct ReflectDepth {
-	static constexpr int AC = is_cplx<T>::value ? 2 : 4;
-	static constexpr int LD = GMEM ? 2 * AC : AC;
+	static constexpr int AC = is_cplx<T>::value ? 8 : 4;
+	static constexpr int LD = is_cplx<T>::value ? (GMEM ? 4 : 2) : (GMEM ? 8 : 4);
 	static constexpr int RT = is_cplx<T>::value ? (GMEM ? 4 : 2) : (GMEM ? 8 : 3);
 };
 
@@ -1301,8 +1299,7 @@ struct RecArgs {
 // G = (D_b^-1 Q^H + D_s T)^-1 D_b^-1 Q^H (greens.c:157-178), or its two-sided
 // form, one CTA per item with M in shared memory (GM: in global memory):
 //   * LU with partial pivoting in panels of 8 columns (getrf; the pivot is the
-//     first largest entry, in modulus for real and by |re| + |im| for complex
-//     scalars, as idamax / izamax).  The panel's warps hold it in registers,
+//     first largest entry, see pivot_mag).  The panel's warps hold it in registers,
 //     rows in place with their positions beside them.  A column costs one
 //     barrier among them: each warp leaves its candidate row in shared memory
 //     before it, and takes the winner's row from there after it.  They write
@@ -1323,9 +1320,18 @@ struct RecArgs {
 // in the diagonal blocks; 512 items 0.75 ms against 1.77; N = 256 (M in L2)
 // 1.09 ms against 6.0; complex N = 100 0.50 ms for 64 items against 1.12.
 
-// the magnitude a pivot is chosen by
+// The magnitude a pivot is chosen by: the modulus, for complex scalars within 8%
+// of it (the octagon's norm; an infinity or a NaN stays one).  |re| + |im|, up to
+// 41% off, lets multipliers grow to 1.41: G of well-conditioned complex products 1
+// to 2% further from the exact one.  hypot as in the unblocked LU costs 10% of
+// the launch at N = 64.
 __device__ inline double pivot_mag(double a) { return fabs(a); }
-__device__ inline double pivot_mag(zd a) { return fabs(a.x) + fabs(a.y); }
+__device__ inline double pivot_mag(zd a)
+{
+	const double x = fabs(a.x), y = fabs(a.y);
+	const bool xl = x >= y;
+	return fma(0.41421356, xl ? y : x, xl ? x : y);
+}
 
 // the warps of a panel: one up to N = 64, else four; up to two rows a lane
 template <int RPL>
@@ -1556,10 +1562,15 @@ __device__ inline void lu_u_rows(T *M, int ld, int N, int j0, int pb, int c0, in
 	tile_c_to_b(u, b, lane);
 }
 
-// M -= L U on the rows from j0 + pb on of the columns c0 .. c0+7, one warp
+// M -= L U on the rows from j0 + pb on of the columns c0 .. c0+7, one warp.  A
+// complex term adds its two real products one after the other, two roundings at
+// M's size where a scalar update has one, so a complex tile sums L U by itself and
+// adds it to M once (N = 100 x 64 257 -> 265 us a launch; G of well-conditioned
+// complex products 3 to 5% closer to the exact one).
 template <typename T>
 __device__ inline void lu_trail(T *M, int ld, int N, int j0, int pb, int c0, const T (&b)[2], int lane)
 {
+	constexpr bool SUM = is_cplx<T>::value;
 	constexpr int RT = is_cplx<T>::value ? 2 : 3;   // row tiles at a time
 	const int lr = lane & 3, lq = lane >> 2, cc = c0 + 2 * lr;
 	for (int r0 = j0 + pb; r0 < N; r0 += 8 * RT) {
@@ -1570,7 +1581,7 @@ __device__ inline void lu_trail(T *M, int ld, int N, int j0, int pb, int c0, con
 		for (int i = 0; i < RT; i++) {
 			const bool in = r0 + 8 * i + lq < N;
 #pragma unroll
-			for (int e = 0; e < 2; e++) x[i][e] = (in && cc + e < N) ? Mx[8 * i + ld * e] : zero<T>();
+			for (int e = 0; e < 2; e++) x[i][e] = (!SUM && in && cc + e < N) ? Mx[8 * i + ld * e] : zero<T>();
 #pragma unroll
 			for (int s = 0; s < 2; s++) a[i][s] = (in && 4 * s + lr < pb) ? -Ma[8 * i + ld * 4 * s] : zero<T>();
 		}
@@ -1583,7 +1594,7 @@ __device__ inline void lu_trail(T *M, int ld, int N, int j0, int pb, int c0, con
 			const bool in = r0 + 8 * i + lq < N;
 #pragma unroll
 			for (int e = 0; e < 2; e++)
-				if (in && cc + e < N) Mx[8 * i + ld * e] = x[i][e];
+				if (in && cc + e < N) Mx[8 * i + ld * e] = SUM ? Mx[8 * i + ld * e] + x[i][e] : x[i][e];
 		}
 	}
 	__syncwarp();

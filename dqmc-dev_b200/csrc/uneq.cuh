@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(NW * 32) k_hqr(HqrArgs<T> a)
 			const int c1 = min(j1 + NBK, n), n1 = n + a.nx1 - c1;
 			const int t1 = (n1 + 7) / 8, t2 = (a.nx2 + 7) / 8, t3 = (M + 7) / 8;
 			using D = ReflectDepth<T, true>;
-			constexpr int AC = D::LD;      // one accumulator per load in flight
+			constexpr int AC = 8;          // of W: M = 2 N rows a sum
 			for (int t = slot; t < t1 + t2 + t3; t += ns) {
 				T *C;
 				size_t ldc = lda;

@@ -716,7 +716,7 @@ struct GroupBase {
 	// events: class sums as profile(), and the kernels it launched
 	virtual int profile_grad(int which, double *out, int ncls, int *launches) = 0;
 	// whether the delayed update holds G on chip (k_update_cl)
-	virtual bool update_on_chip() = 0;
+	virtual int update_on_chip() = 0;
 	// the eight hopping matrices exp(-+dt K), exp(-+dt K / 2) of both spins
 	virtual int set_hopping(const void *const *m) = 0;
 	// G drift self-check: on / off (resets the counters when turned on), and
@@ -2017,9 +2017,8 @@ struct Group : GroupBase, ProfHook {
 		precs.clear();
 	}
 
-	// whether the choice between the update's two forms fell on k_update_cl:
-	// it is offered where one spin's G fits one SM
-	bool update_on_chip() override { return upd_split > 0 && update_cl_split<T>(N, kd, 1) == 1; }
+	// 0: k_update; k_update_cl: 1 where one SM holds one spin's G, else 2
+	int update_on_chip() override { return !upd_split ? 0 : update_cl_split<T>(N, kd, 1) == 1 ? 1 : 2; }
 
 	int profile_grad(int which, double *out, int ncls, int *launches) override
 	{
@@ -2627,7 +2626,7 @@ struct Lanes : GroupBase {
 		return 0;
 	}
 
-	bool update_on_chip() override { return g[0]->update_on_chip(); }
+	int update_on_chip() override { return g[0]->update_on_chip(); }
 
 	// class sums and launches over the lanes, each profiled alone
 	int profile_grad(int which, double *out, int ncls, int *launches) override
@@ -3089,7 +3088,7 @@ int dqmc_engine_profile_sweep(dqmc_engine *e, int meas_eq, int meas_ue, double *
 
 int dqmc_engine_update_on_chip(dqmc_engine *e)
 {
-	return e ? (e->g->update_on_chip() ? 1 : 0) : DQMC_E_ARG;
+	return e ? e->g->update_on_chip() : DQMC_E_ARG;
 }
 
 int dqmc_engine_profile_grad(dqmc_engine *e, int which, double *out, int n_class, int *launches)

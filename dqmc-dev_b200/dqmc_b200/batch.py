@@ -20,8 +20,7 @@ files' value.  `autotune` also times every group of 32 chains or more in
 fastest, and for each lattice size it times the delayed update's two forms
 on the first group of that size: G in device memory with one CTA per chain
 (k_update), or G on chip in a cluster of CTAs per chain (k_update_cl), where
-one spin's G and panels fit in one SM's shared memory; larger lattices keep
-the engine's rule.  Neither lanes nor the update form change results.
+one spin's G and panels fit in the shared memory of up to four SMs.  Neither lanes nor the update form change results.
 """
 from __future__ import annotations
 
@@ -71,13 +70,15 @@ def time_sweep(sims: list[SimData], n_delay: int | None, device: int = 0,
         e.close()
 
 
-def update_forms(sims: list[SimData], n_delay: int | None = None, device: int = 0) -> list[str]:
-    """The delayed-update forms to choose from for these chains: "global"
-    always, "cluster" where one spin's G and panels fit in one SM's shared
-    memory."""
+def update_forms(sims: list[SimData], n_delay: int | None = None, device: int = 0,
+                 spread: bool = False) -> list[str]:
+    """The delayed-update forms of these chains: "global" always, "cluster"
+    where one spin's G and panels fit in one SM's shared memory, with `spread`
+    also where they take that of two or four."""
     e = Engine([sims[0].clone()], device=device, n_delay=n_delay, update="cluster")
     try:
-        return ["global", "cluster"] if e.update_form == "cluster" else ["global"]
+        r = e.lib.dqmc_engine_update_on_chip(e.h)
+        return ["global", "cluster"] if r == 1 or (spread and r > 1) else ["global"]
     finally:
         e.close()
 
@@ -87,7 +88,7 @@ def autotune_update(sims: list[SimData], device: int = 0, n_delay: int | None = 
     """The delayed-update form ("global" or "cluster") with the shorter
     timed sweeps of copies of all of `sims`.  Both forms do the same
     arithmetic in the same order, so the choice only changes the speed."""
-    forms = update_forms(sims, n_delay, device)
+    forms = update_forms(sims, n_delay, device, spread=True)
     if len(forms) == 1:
         return forms[0]
     t = {f: time_sweep(sims, n_delay, device, lanes=lanes, update=f, n=2) for f in forms}
@@ -159,11 +160,9 @@ class RaggedBatch:
             for g, idx in enumerate(self.groups):
                 n = sims[idx[0]].N
                 if n not in self.update:
-                    group = [sims[i] for i in idx]
-                    # where there is no choice the engine's own rule stands
-                    self.update[n] = None if len(update_forms(group, self.delay.get(n), device)) == 1 \
-                        else autotune_update(group, device=device, n_delay=self.delay.get(n),
-                                             lanes=self.lanes.get(g))
+                    self.update[n] = autotune_update([sims[i] for i in idx], device=device,
+                                                     n_delay=self.delay.get(n),
+                                                     lanes=self.lanes.get(g))
         self.engines = [Engine([sims[i] for i in idx], device=device,
                                n_delay=self.delay.get(sims[idx[0]].N), lanes=self.lanes.get(g),
                                update=self.update.get(sims[idx[0]].N))

@@ -265,12 +265,11 @@ class Engine:
 
     @property
     def update_form(self) -> str:
-        """"cluster" when the delayed update holds G on chip (k_update_cl)
-        and one SM per spin would do, else "global"
-        (dqmc_engine_update_on_chip)."""
+        """"cluster" when the delayed update holds G on chip (k_update_cl),
+        else "global" (dqmc_engine_update_on_chip)."""
         r = self.lib.dqmc_engine_update_on_chip(self.h)
         _lib.check(min(r, 0), "dqmc_engine_update_on_chip")
-        return "cluster" if r == 1 else "global"
+        return "cluster" if r > 0 else "global"
 
     def profile_grad(self, which: str, n_class: int = 7):
         """One gradient evaluation ("logdet" or "obs") with per-launch CUDA

@@ -155,16 +155,15 @@ int dqmc_engine_accepts(dqmc_engine *e, int chain, long long *n);
 /* CUDA stream the engine queues on, as an opaque handle (cudaStream_t):
  * every sweep forks from it to the lanes' streams and joins back to it */
 void *dqmc_engine_stream(dqmc_engine *e);
-/* 1 when the engine's delayed update holds each spin's G in the shared memory
- * of one SM or more (k_update_cl: a cluster of two, four or eight CTAs per
- * chain) and one SM would do; 0 when G stays in device memory (k_update), and
- * for the lattices whose G only fits the shared memory of several SMs, which
- * take k_update_cl unless DQMC_UPDATE=global.  All give bit-identical results.
- * Chosen at creation: DQMC_UPDATE=cluster or =global when set, else on chip
- * for N >= 25 with at most 74 chains, or with any number of chains from
- * N = 128 (complex: 90) up, where one spin's G and panels fit the shared
- * memory of four SMs.  dqmc_gpu_update_delayed applies the same rule to its
- * batch. */
+/* the form of the engine's delayed update: 0 when G stays in device memory
+ * (k_update), positive when it lies in shared memory (k_update_cl: a cluster of
+ * two, four or eight CTAs per chain, half of them per spin): 1 where one SM
+ * would hold one spin's G and panels, 2 where it takes two or four.  All give
+ * bit-identical results.  Chosen at creation: DQMC_UPDATE=cluster or =global
+ * when set, else on chip for N >= 25 with at most 74 chains, or with any number
+ * of chains from N = 128 (complex: 90) up, where one spin's G and panels fit the
+ * shared memory of four SMs.  dqmc_gpu_update_delayed applies the same rule to
+ * its batch. */
 int dqmc_engine_update_on_chip(dqmc_engine *e);
 /* number of kernels one sweep of the given kind launches */
 int dqmc_engine_launches_per_sweep(dqmc_engine *e, int meas_eq, int meas_ue);

@@ -613,51 +613,19 @@ __global__ void k_rotate_slices(int N, int L, int NB, int s, const double *src, 
 	}
 }
 
-// The delayed update runs as one CTA per chain with G in device memory
-// (k_update), or with G held in shared memory by a cluster of 2 P CTAs per
-// chain, P per spin (k_update_cl).  Both do the same arithmetic in the same
-// order.  The on-chip form shortens a slice but a chain then holds 2 P SMs, so
-// the rule goes by what fits at once and by what that gains.  Microseconds per
-// slice, device memory / P = 1 / 2 / 4 (real, then complex scalars):
-//   N = 16,    1 chain     16 /  17 /  17 /  18
-//   N = 64,    1 chain     44 /  39 /  38 /  39      103 /  80 /  74 /  73
-//   N = 64,   32 chains    47 /  41 /  40 / 100      112 /  87 /  81 / 198
-//   N = 64,  128 chains    48 /  73 / 137 / 296      114 / 162 / 286 / 602
-//   N = 100,   8 chains   108 /  75 /  67 /  63      290 /   - / 154 / 140
-//   N = 144,  32 chains   226 / 108 /  97 / 239
-//   N = 144, 256 chains   448 / 400 / 708 / 1422
-// More than one CTA per spin pays from N = 90 up (complex: 64), while the
-// clusters find room side by side: 2 P chains <= 128 CTAs for P = 2, half of
-// that for clusters of eight.  Beyond one wave of CTAs (74 chains) only the
-// larger lattices keep the on-chip form.  DQMC_UPDATE=cluster or =global
-// overrides the choice between the two forms (read when an engine is created,
-// or a seam called).  0: G in device memory, else P.
 template <typename T>
-static int update_split(int N, int kd, int chains)
-{
-	constexpr bool CX = is_cplx<T>::value;
-	const char *v = getenv("DQMC_UPDATE");
-	const bool cl = (v && *v) ? strcmp(v, "cluster") == 0
-	                          : N >= 25 && (chains <= 74 || N >= (CX ? 90 : 128));
-	if (!cl || N > 480) return 0;
-	const int p = (N >= 90 && chains <= 8) ? 4 : (N >= (CX ? 64 : 90) && chains <= 32) ? 2 : 1;
-	return update_cl_split<T>(N, kd, p);
-}
-
-template <typename T>
-static cudaError_t update_attr(int N, int kd, int ldp, int split)
+static cudaError_t update_attr(int N, int kd, int ldp, int split, int chains)
 {
 	if (split) return raise_smem(k_update_cl<T>, update_cl_smem_bytes<T>(N, split, kd));
-	const cudaError_t er = raise_smem(k_update<T>, update_smem_bytes<T>(N, kd, ldp));
-	return er != cudaSuccess ? er : raise_smem(k_update_big<T>, update_smem_bytes<T>(N, kd, ldp));
+	return raise_smem(update_kernel<T>(N, chains), update_smem_bytes<T>(N, kd, ldp));
 }
 
 // the delayed update of a.nchain chains: on chip (split > 0), a cluster of
 // 2 split CTAs of cl_warps(N) warps and one look-ahead warp per chain; else one
-// CTA of update_warps(N) warps and one look-ahead warp per chain, in the launch
-// form sized for that CTA
+// CTA of update_warps(N) warps and one look-ahead warp per chain, in the instance
+// for that CTA and the engine's chains
 template <typename T>
-static int launch_update(const UpdArgs<T> &a, cudaStream_t st, int split)
+static int launch_update(const UpdArgs<T> &a, cudaStream_t st, int split, int chains)
 {
 	cudaLaunchConfig_t cfg = {};
 	cudaLaunchAttribute at = {};
@@ -677,7 +645,7 @@ static int launch_update(const UpdArgs<T> &a, cudaStream_t st, int split)
 		cfg.gridDim = dim3(a.nchain);
 		cfg.blockDim = dim3(update_warps(a.N) * 32 + 32);
 		cfg.dynamicSmemBytes = update_smem_bytes<T>(a.N, a.n_delay, a.ldp);
-		e = cudaLaunchKernelEx(&cfg, cfg.blockDim.x <= 352 ? k_update<T> : k_update_big<T>, a);
+		e = cudaLaunchKernelEx(&cfg, update_kernel<T>(a.N, chains), a);
 	}
 	if (e == cudaSuccess) return 0;
 	fprintf(stderr, "dqmc_b200: update launch failed: %s\n", cudaGetErrorString(e));
@@ -748,6 +716,7 @@ struct Group : GroupBase, ProfHook {
 	int N, L, F, nmul;
 	int sweep = 0;
 	int kd = 0, ldp = 0;   // delayed-update flush period and panel ld
+	int upd_chains = 0;    // chains of the engine this group is a lane of
 	int upd_split = 0;     // CTAs per spin of the on-chip delayed update, 0: G in device memory
 	int eq_size = 0, ue_size = 0;
 	cudaStream_t st = nullptr;
@@ -962,8 +931,9 @@ struct Group : GroupBase, ProfHook {
 		return p.meas_gen_suscept || p.meas_chiral || p.meas_energy_corr || p.meas_local_JQ;
 	}
 
-	// nchain chains of an engine of engine_chains (the update form's rule)
-	int create(const dqmc_params &pp, int nchain, int engine_chains)
+	// nchain chains, a lane of an engine of engine_chains whose largest lane has
+	// lane_chains (the update form's rule)
+	int create(const dqmc_params &pp, int nchain, int lane_chains, int engine_chains)
 	{
 		p = pp;
 		C = nchain;
@@ -1037,8 +1007,9 @@ struct Group : GroupBase, ProfHook {
 		// delayed-update panels: the file's n_delay unless shared memory is short
 		ldp = (N + 15) / 16 * 16 + 4;
 		kd = update_delay<T>(N, p.n_delay, ldp);
-		upd_split = update_split<T>(N, kd, engine_chains);
-		CK(update_attr<T>(N, kd, ldp, upd_split));
+		upd_split = update_split<T>(N, kd, lane_chains, engine_chains);
+		CK(update_attr<T>(N, kd, ldp, upd_split, engine_chains));
+		upd_chains = engine_chains;
 		CK(cudaDeviceSynchronize());
 		return 0;
 	}
@@ -1462,7 +1433,7 @@ struct Group : GroupBase, ProfHook {
 		// slice again (L = 1), whose fields this kernel is still changing
 		a.next_slice = (L == 1) ? -1 : (l + 1) % L;
 		prof_begin(1);
-		if (const int rc = launch_update<T>(a, st, upd_split)) return rc;
+		if (const int rc = launch_update<T>(a, st, upd_split, upd_chains)) return rc;
 		prof_end(PC_UPDATE, 0.0, 0.0);
 		launch_count++;
 		watchdog("k_update");
@@ -2457,11 +2428,11 @@ struct Lanes : GroupBase {
 			int rc;
 			if (p.cplx) {
 				auto *gg = new Group<zd>();
-				rc = gg->create(p, n, n_chain);
+				rc = gg->create(p, n, (n_chain + n_lane - 1) / n_lane, n_chain);
 				x = gg;
 			} else {
 				auto *gg = new Group<double>();
-				rc = gg->create(p, n, n_chain);
+				rc = gg->create(p, n, (n_chain + n_lane - 1) / n_lane, n_chain);
 				x = gg;
 			}
 			if (rc) {
@@ -3140,8 +3111,8 @@ static int seam_update(int batch, int N, int n_delay, const double *del, uint64_
 	if (batch < 1 || N < 1 || N > 480 || n_delay < 1 || !del || !rng || !hs || !G || !phase)
 		return DQMC_E_ARG;
 	const int ldp = (N + 15) / 16 * 16 + 4, kd = update_delay<T>(N, n_delay, ldp);
-	const int split = update_split<T>(N, kd, batch);
-	CK(update_attr<T>(N, kd, ldp, split));
+	const int split = update_split<T>(N, kd, batch, batch);
+	CK(update_attr<T>(N, kd, ldp, split, batch));
 	Slab sc;
 	uint64_t *ck;
 	int *ord;
@@ -3157,7 +3128,7 @@ static int seam_update(int batch, int N, int n_delay, const double *del, uint64_
 	a.N = N; a.L = 1; a.n_delay = kd; a.nchain = batch; a.slice = 0; a.ldp = ldp;
 	a.del = del; a.rng = rng; a.rng_ckpt = ck; a.hs = hs; a.G = (T *)G; a.phase = (T *)phase;
 	a.order = ord; a.u = uu; a.next_slice = -1; a.err = err;
-	const int rc = launch_update<T>(a, st, split);
+	const int rc = launch_update<T>(a, st, split, batch);
 	unsigned e = 0;
 	CK(cudaMemcpyAsync(&e, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));

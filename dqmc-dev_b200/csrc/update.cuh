@@ -704,19 +704,37 @@ __device__ __forceinline__ void update_chain(const UpdArgs<T> &a)
 	}
 }
 
-// k_update bounds the registers so that two CTAs of N <= 160 share an SM when
-// there are more chains than SMs (real scalars); k_update_big takes the larger
-// CTAs
-template <typename T>
-__global__ void __launch_bounds__(352, is_cplx<T>::value ? 1 : 2) k_update(UpdArgs<T> a)
+// MAXT threads, MINB CTAs on an SM.  While every chain has an SM to itself, CTAs
+// take the registers they want; with more chains than SMs the small ones leave
+// room for a second CTA as long as that does not cost many spills (real N <= 128; with
+// room for two CTAs of 352 threads the bound is 80 registers).  Microseconds a
+// slice, one CTA / two: real N = 64 x 256 chains - / 77 (154 registers either way),
+// N = 81 x 128 97 / 109, x 256 186 / 136, N = 100 x 128 117 / 154, x 256 229 / 204,
+// N = 144 x 32 234 / 359, x 256 477 / 577; complex N = 64 x 128 112 / 123, x 256
+// 227 / 151.
+template <typename T, int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) k_update(UpdArgs<T> a)
 {
 	update_chain(a);
 }
 
+// k_update's instance for N's CTA; chains: those of the whole engine, whose lanes
+// share the SMs
 template <typename T>
-__global__ void __launch_bounds__(480, 1) k_update_big(UpdArgs<T> a)
+auto update_kernel(int N, int chains)
 {
-	update_chain(a);
+	const int t = update_warps(N) * 32 + 32;
+	const bool one = chains <= 148;
+	if constexpr (is_cplx<T>::value) {
+		if (t <= 160 && one) return k_update<T, 160, 1>;
+		// 168 registers: two CTAs of 160 threads fit as well
+		return t <= 352 ? k_update<T, 352, 1> : k_update<T, 480, 1>;
+	} else {
+		if (t <= 160) return k_update<T, 160, 2>;
+		if (t <= 224 && !one) return k_update<T, 224, 2>;
+		if (t <= 288 && !one) return k_update<T, 288, 2>;
+		return t <= 352 ? k_update<T, 352, 1> : k_update<T, 480, 1>;
+	}
 }
 
 }  // namespace dq

@@ -35,6 +35,9 @@
 // (G in device memory 468), N = 256 - / - / 182 (935).
 #pragma once
 
+#include <cstdlib>
+#include <cstring>
+
 #include "mbar.cuh"
 #include "update.cuh"
 
@@ -307,6 +310,56 @@ template <typename T>
 size_t update_cl_smem_bytes(int N, int P, int kd)
 {
 	return cl_plan<T>(N, P, kd).total;
+}
+
+// The form of the delayed update: 0 for one CTA per chain with G in device memory
+// (k_update), else the CTAs per spin P of k_update_cl.  Both do the same arithmetic
+// in the same order.  The on-chip form shortens a slice but a chain then holds 2 P
+// SMs (74, 36 and 15 clusters run at once for P = 1, 2, 4), so the rule goes by what
+// runs at once and by how much that gains.  launch: the chains of the largest
+// launch, chains: those of all lanes.  Milliseconds a sweep of L = 10 in the
+// default lanes, device memory / the fewest SMs that hold G:
+//                    32        64       100       128       192       256 chains
+//   real  N = 36  .66/.55   .70/.59   .76/.66   .84/.72  1.00/.93  1.28/1.21
+//             64 1.06/.78  1.11/.84  1.33/1.37 1.36/1.26 1.76/1.74 2.30/2.52
+//            100 2.03/1.59 2.27/1.84 3.09/3.32 3.15/3.12 4.67/4.49 5.71/6.03
+//            121 2.94/2.07 3.42/2.56 4.47/4.41 4.62/4.25 7.14/6.26 8.86/8.36
+//            144 3.90/2.56 4.32/3.00 5.80/5.45 5.97/5.28 8.42/7.75 11.3/10.3
+//   P = 2    156 5.13/3.57 5.63/5.07 7.90/9.32 8.54/9.82 12.3/14.4 19.6/21.9
+//            196 8.13/5.18 9.60/8.20 13.4/15.0 15.4/16.3 22.5/24.1 31.8/32.7
+//   P = 4    225 14.0/11.4 16.6/17.0 23.7/27.3 26.8/31.2 39.8/46.3 52.4/61.0
+//            256 17.6/13.6 20.5/20.1 29.6/31.9 33.6/36.0 48.7/53.3 65.8/70.7
+//   cplx      25  .60/.62   .64/.66   .76/.81   .83/.91  1.07/1.16 1.32/1.44
+//             36 1.02/.91  1.12/.98  1.32/1.26 1.51/1.42 1.99/1.97 2.44/2.50
+//             64 1.88/1.54 2.12/1.77 2.52/2.41 2.85/2.95 3.91/4.40 4.63/5.72
+//             81 3.45/2.57 3.91/3.07 4.62/4.18 5.16/5.12 7.10/7.57 9.28/10.0
+//   P = 2    100 4.66/3.56 5.34/5.43 6.47/8.18 7.61/10.2 11.0/15.4 14.6/20.4
+//            121 6.62/4.81 8.31/7.93 9.74/11.6 12.5/15.2 16.7/21.4 21.9/28.4
+//   P = 4    144 9.20/9.97 11.5/15.1 (16 chains 8.34/7.24)
+//            169 16.1/14.7 20.0/21.6
+// More than one CTA per spin where one would do pays from N = 90 up (complex: 64)
+// while the clusters run at once: 8 chains real N = 100 1.39 / 1.32 / 1.28 ms for P
+// = 1 / 2 / 4, 32 chains 1.59 / 1.52 / 2.55.  DQMC_UPDATE=cluster or =global
+// overrides the choice between the two forms (read when an engine is created, or a
+// seam called).
+template <typename T>
+int update_split(int N, int kd, int launch, int chains)
+{
+	constexpr bool CX = is_cplx<T>::value;
+	const char *v = getenv("DQMC_UPDATE");
+	const bool forced = v && *v;
+	if (N > 480 || (forced ? strcmp(v, "cluster") != 0 : N < (CX ? 30 : 25))) return 0;
+	const int pmin = update_cl_split<T>(N, kd, 1);
+	if (!pmin) return 0;
+	if (!forced) {
+		int limit;      // chains beyond which G in device memory is faster
+		if (pmin == 1) limit = CX ? (N < 56 ? chains : 110) : (N < 64 || N >= 112) ? chains : launch <= 74 ? 222 : 74;
+		else if (pmin == 2) limit = CX && N < 112 ? 36 : 72;
+		else limit = !CX ? 60 : N < 160 ? 30 : 45;
+		if (chains > limit) return 0;
+	}
+	const int p = (N >= 90 && chains <= 8) ? 4 : (N >= (CX ? 64 : 90) && chains <= 32) ? 2 : 1;
+	return update_cl_split<T>(N, kd, p);
 }
 
 }  // namespace dq

@@ -160,10 +160,11 @@ void *dqmc_engine_stream(dqmc_engine *e);
  * two, four or eight CTAs per chain, half of them per spin): 1 where one SM
  * would hold one spin's G and panels, 2 where it takes two or four.  All give
  * bit-identical results.  Chosen at creation: DQMC_UPDATE=cluster or =global
- * when set, else on chip for N >= 25 with at most 74 chains, or with any number
- * of chains from N = 128 (complex: 90) up, where one spin's G and panels fit the
- * shared memory of four SMs.  dqmc_gpu_update_delayed applies the same rule to
- * its batch. */
+ * when set, else by N and the number of chains, on chip where one spin's G and
+ * panels fit the shared memory of four SMs and the clusters that run at once
+ * outweigh what they gain (real N >= 25, complex N >= 30, up to 110 chains or more
+ * where one SM holds a spin's G, 30 to 72 where it takes several).
+ * dqmc_gpu_update_delayed applies the same rule to its batch. */
 int dqmc_engine_update_on_chip(dqmc_engine *e);
 /* number of kernels one sweep of the given kind launches */
 int dqmc_engine_launches_per_sweep(dqmc_engine *e, int meas_eq, int meas_ue);

@@ -99,8 +99,10 @@ __device__ inline zd warp_sum(zd v) {
 
 // Warp-level FP64 tensor-core MMA, m8n8k4 (row-major A 8x4, col-major B 4x8):
 // lane l holds a = A[l/4][l%4], b = B[l%4][l/4], c = C[l/4][2(l%4)+{0,1}].
+// Volatile: all lanes take part, so it must not move under a lane's test of its
+// results (launches take the same time without).
 __device__ inline void dmma(double &c0, double &c1, double a, double b) {
-	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+	asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
 	             : "+d"(c0), "+d"(c1)
 	             : "d"(a), "d"(b));
 }

@@ -35,6 +35,10 @@ import ctypes as C
 from . import lib as _lib
 from .engine import INT_PARAMS, Engine, SimData
 
+# accepts after which a window of the delayed update is flushed at the latest: a
+# larger n_delay acts as this one
+MAX_DELAY = 16
+
 # parameters a group shares (everything except U's exp_lambda and del)
 _SHARED_ARRAYS = ("map_i", "map_ij", "bonds", "map_bb", "peierlsu", "peierlsd")
 
@@ -114,12 +118,15 @@ def autotune_lanes(sims: list[SimData], candidates=(1, 2, 4, 8), device: int = 0
 def autotune_delay(sims: list[SimData], candidates=(4, 8, 16, 32), device: int = 0,
                    max_chains: int = 8) -> int:
     """The candidate delay rank with the shortest timed sweep of (up to
-    max_chains of) these chains; candidates a chain cannot use are skipped."""
+    max_chains of) these chains; candidates a chain cannot use are skipped, and
+    those that act as an earlier one (MAX_DELAY)."""
     probe = sims[:max_chains]
     best, best_t = None, None
+    seen = set()
     for kd in candidates:
-        if kd > probe[0].N:
+        if kd > probe[0].N or min(kd, MAX_DELAY) in seen:
             continue
+        seen.add(min(kd, MAX_DELAY))
         t = time_sweep(probe, kd, device)
         if best_t is None or t < best_t:
             best, best_t = kd, t

@@ -15,6 +15,12 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200, sm_100a)")
 
 
+def pytest_collection_modifyitems(items):
+    """The long runs fail where the reference's own build (oracle/_ref) is absent:
+    last, so that a run that stops at the first failure has run all others."""
+    items.sort(key=lambda it: it.path.name == "test_gpu_longrun.py")
+
+
 @pytest.fixture(scope="session", autouse=True)
 def _oracle_built():
     """Build the CPU oracle once per session (it is a few seconds of gcc)."""

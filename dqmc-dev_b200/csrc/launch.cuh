@@ -41,7 +41,7 @@ bool tma_map_operand(CUtensorMap *map, int *tz, int *tw, const void *base, int e
 // matrix in the caller's per-item workspace, L2-resident) up to 256
 template <typename T> constexpr int max_dense_n() { return 256; }
 
-// batched GEMM in the mode g.mode, tile chosen by least padded area
+// batched GEMM in the mode g.mode
 template <typename T> int launch_gemm(const GemmArgs<T> &g, cudaStream_t st);
 // pre-sorted (QR_PRESORT) and column-pivoted (QR_PIVOT) QR with explicit Q
 template <typename T> int launch_qr_presort(const QrArgs<T> &a, cudaStream_t st);

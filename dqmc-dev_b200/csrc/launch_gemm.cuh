@@ -75,23 +75,45 @@ static int launch_gemm_cfg(const GemmArgs<T> &g, cudaStream_t st)
 // 3.8 / 5.6 / 9.5, x 16 8.7 / 7.1 / 9.6, x 64 21.7 / 20.7 / 16.3; complex
 // N = 100 x 2 4.8 / 8.8 / 19.3, x 32 15.4 / 18.6 / 19.4.  The lines lie where
 // the next tile overtakes: about 1000 CTAs of 16 x 16 (complex 1600), 600 of
-// 32 x 32 (real).  Beyond, the least padded area counts, larger tiles on ties; the 56
-// and 40 tiles (one warp per 8 columns) are for the sizes between 64 and 48:
-// N = 100 x 512 53.5 us (64: 69.7), N = 196 x 512 260 (32: 346), N = 75 x 512
-// 30.9 (48: 35.9), complex N = 100 x 128 57.4 (64: 65.6).
+// 32 x 32 (real).  Beyond, the padded area counts, times what a tile takes for
+// its area (percent of a 64 tile's, gemm_tile_cost), larger tiles on ties.  The 56
+// and 40 tiles (one warp per 8 columns) are for the sizes between 64 and 48 and for
+// matrices that are at least narrow: N = 100 x 512 53 us (64: 69), N = 196 x 256 137
+// (32: 178), N = 75 x 512 31 (48: 35), complex N = 100 x 512 191 (64: 217).  A large
+// matrix of few CTAs shows their long k-steps (N = 1000 x 1: 99 us against 70 with
+// 48, complex 360 against 248), and complex 40 tiles pay from a fifth less area
+// on (N = 156 x 512 550 us against 488 with 32, N = 196 x 256 548 against 591).
+inline int gemm_tile_cost(bool cplx, int t)
+{
+	switch (t) {
+	case 56: return 108;
+	case 40: return cplx ? 120 : 102;
+	case 32: return cplx ? 100 : 103;
+	default: return 100;
+	}
+}
+
+inline int gemm_tile(bool cplx, int batch, int M, int N)
+{
+	auto tiles = [&](int t) { return (long long)((M + t - 1) / t) * ((N + t - 1) / t); };
+	if (batch * tiles(16) <= (cplx ? 1600 : 1024)) return 16;
+	if (!cplx && batch * tiles(32) <= 600) return 32;
+	auto cost = [&](int t) { return tiles(t) * t * t * gemm_tile_cost(cplx, t); };
+	int best = 64;
+	for (int t : {56, 48, 40, 32}) {
+		if ((t == 56 || t == 40) && M > 256 && N > 256) continue;
+		if (cost(t) < cost(best)) best = t;
+	}
+	return best;
+}
+
 template <typename T>
 int launch_gemm(const GemmArgs<T> &g, cudaStream_t st)
 {
 	// the scale vectors and gather indices of these modes are staged per K
 	const bool k_staged = g.mode & (GM_A_DD | GM_B_ROWD | GM_B_GATHER);
 	if ((k_staged && g.K > 512) || g.M < 1 || g.N < 1 || g.K < 1 || g.batch < 1) return DQMC_E_ARG;
-	auto pad = [&](int t) { return (long long)((g.M + t - 1) / t * t) * ((g.N + t - 1) / t * t); };
-	int best = 64;
-	for (int t : {56, 48, 40, 32})
-		if (pad(t) < pad(best)) best = t;
-	auto ctas = [&](int t) { return (long long)g.batch * ((g.M + t - 1) / t) * ((g.N + t - 1) / t); };
-	if (ctas(16) <= (is_cplx<T>::value ? 1600 : 1024)) best = 16;
-	else if (!is_cplx<T>::value && ctas(32) <= 600) best = 32;
+	const int best = gemm_tile(is_cplx<T>::value, g.batch, g.M, g.N);
 	if constexpr (is_cplx<T>::value) {
 		switch (best) {
 		case 64: return launch_gemm_cfg<T, 64, 64, 8, 4, 2, 3>(g, st);

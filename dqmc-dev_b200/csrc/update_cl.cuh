@@ -329,7 +329,7 @@ size_t update_cl_smem_bytes(int N, int P, int kd)
 //            196 8.13/5.18 9.60/8.20 13.4/15.0 15.4/16.3 22.5/24.1 31.8/32.7
 //   P = 4    225 14.0/11.4 16.6/17.0 23.7/27.3 26.8/31.2 39.8/46.3 52.4/61.0
 //            256 17.6/13.6 20.5/20.1 29.6/31.9 33.6/36.0 48.7/53.3 65.8/70.7
-//   cplx      25  .60/.62   .64/.66   .76/.81   .83/.91  1.07/1.16 1.32/1.44
+//   cplx      32  .67/.69   .71/.74   .83/.88   .93/.98  1.21/1.26 1.52/1.58
 //             36 1.02/.91  1.12/.98  1.32/1.26 1.51/1.42 1.99/1.97 2.44/2.50
 //             64 1.88/1.54 2.12/1.77 2.52/2.41 2.85/2.95 3.91/4.40 4.63/5.72
 //             81 3.45/2.57 3.91/3.07 4.62/4.18 5.16/5.12 7.10/7.57 9.28/10.0
@@ -348,7 +348,7 @@ int update_split(int N, int kd, int launch, int chains)
 	constexpr bool CX = is_cplx<T>::value;
 	const char *v = getenv("DQMC_UPDATE");
 	const bool forced = v && *v;
-	if (N > 480 || (forced ? strcmp(v, "cluster") != 0 : N < (CX ? 30 : 25))) return 0;
+	if (N > 480 || (forced ? strcmp(v, "cluster") != 0 : N < (CX ? 33 : 25))) return 0;
 	const int pmin = update_cl_split<T>(N, kd, 1);
 	if (!pmin) return 0;
 	if (!forced) {

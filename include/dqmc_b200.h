@@ -162,7 +162,7 @@ void *dqmc_engine_stream(dqmc_engine *e);
  * bit-identical results.  Chosen at creation: DQMC_UPDATE=cluster or =global
  * when set, else by N and the number of chains, on chip where one spin's G and
  * panels fit the shared memory of four SMs and the clusters that run at once
- * outweigh what they gain (real N >= 25, complex N >= 30, up to 110 chains or more
+ * outweigh what they gain (real N >= 25, complex N >= 33, up to 110 chains or more
  * where one SM holds a spin's G, 30 to 72 where it takes several).
  * dqmc_gpu_update_delayed applies the same rule to its batch. */
 int dqmc_engine_update_on_chip(dqmc_engine *e);

@@ -182,6 +182,48 @@ d 256 100 29.56 - - 31.94
 d 256 128 33.58 - - 35.97
 d 256 192 48.71 - - 53.26
 d 256 256 65.82 - - 70.68
+zd 28 8 0.61 0.71 - -
+zd 28 32 0.63 0.70 - -
+zd 28 64 0.66 0.75 - -
+zd 28 100 0.78 0.88 - -
+zd 28 128 0.87 1.00 - -
+zd 28 192 1.13 1.25 - -
+zd 28 256 1.40 1.55 - -
+zd 30 8 0.65 0.67 - -
+zd 30 32 0.66 0.69 - -
+zd 30 64 0.70 0.74 - -
+zd 30 100 0.82 0.90 - -
+zd 30 128 0.92 1.00 - -
+zd 30 192 1.19 1.26 - -
+zd 30 256 1.45 1.59 - -
+zd 32 8 0.65 0.67 - -
+zd 32 32 0.67 0.69 - -
+zd 32 64 0.71 0.74 - -
+zd 32 100 0.83 0.88 - -
+zd 32 128 0.93 0.98 - -
+zd 32 192 1.21 1.26 - -
+zd 32 256 1.52 1.58 - -
+zd 33 8 0.93 0.82 - -
+zd 33 32 0.98 0.87 - -
+zd 33 64 1.08 0.95 - -
+zd 33 100 1.27 1.21 - -
+zd 33 128 1.43 1.34 - -
+zd 33 192 1.87 1.84 - -
+zd 33 256 2.39 2.41 - -
+d 20 8 0.34 0.35 - -
+d 20 32 0.36 0.36 - -
+d 20 64 0.37 0.38 - -
+d 20 100 0.42 0.43 - -
+d 20 128 0.43 0.45 - -
+d 20 192 0.51 0.53 - -
+d 20 256 0.62 0.66 - -
+d 30 8 0.44 0.42 - -
+d 30 32 0.46 0.43 - -
+d 30 64 0.48 0.46 - -
+d 30 100 0.54 0.54 - -
+d 30 128 0.55 0.54 - -
+d 30 192 0.66 0.67 - -
+d 30 256 0.78 0.78 - -
 """
 
 

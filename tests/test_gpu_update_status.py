@@ -2,9 +2,9 @@
 with an error instead of a sweep without its update, and an error word that the
 kernel has set (a wait that ran out) reaches the seam's caller.
 
-Both come from a fake: the library's objects are linked once more with two calls
-of the runtime wrapped, and when they are told to, the launch returns an error
-code without launching and the copy of an error word to the host brings one.
+Both come from a fake: the library's objects are linked once more with calls of
+the runtime wrapped, and when they are told to, the launch returns an error code
+without launching and the wait finds the error word set.
 """
 import ctypes as C
 import glob
@@ -36,16 +36,24 @@ cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *
 	}
 	return __real_cudaLaunchKernelExC(c, f, a);
 }
-unsigned fake_word = 0;   /* the error word the next 4-byte copy to the host brings */
-cudaError_t __real_cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t st);
-cudaError_t __wrap_cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind k, cudaStream_t st)
+unsigned fake_word = 0;   /* what the next wait on a stream leaves in the call's error word */
+static unsigned *word;
+cudaError_t __real_cudaHostAlloc(void **p, size_t n, unsigned flags);
+cudaError_t __wrap_cudaHostAlloc(void **p, size_t n, unsigned flags)
 {
-	if (fake_word && n == sizeof(unsigned) && k == cudaMemcpyDeviceToHost) {
-		*(unsigned *)d = fake_word;
+	const cudaError_t e = __real_cudaHostAlloc(p, n, flags);
+	if (e == cudaSuccess && n == sizeof(unsigned)) word = (unsigned *)*p;
+	return e;
+}
+cudaError_t __real_cudaStreamSynchronize(cudaStream_t st);
+cudaError_t __wrap_cudaStreamSynchronize(cudaStream_t st)
+{
+	const cudaError_t e = __real_cudaStreamSynchronize(st);
+	if (fake_word && word) {
+		*word |= fake_word;
 		fake_word = 0;
-		return cudaSuccess;
 	}
-	return __real_cudaMemcpyAsync(d, s, n, k, st);
+	return e;
 }
 }
 """
@@ -63,7 +71,8 @@ def fake(tmp_path_factory):
     (d / "fake.cu").write_text(FAKE)
     so = str(d / "libfake.so")
     subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-cudart", "static",
-                    "-Xcompiler", "-fPIC", "-Xlinker", "--wrap=cudaLaunchKernelExC", "-Xlinker", "--wrap=cudaMemcpyAsync", "-o", so,
+                    "-Xcompiler", "-fPIC", "-Xlinker", "--wrap=cudaLaunchKernelExC", "-Xlinker", "--wrap=cudaHostAlloc", "-Xlinker",
+                    "--wrap=cudaStreamSynchronize", "-o", so,
                     str(d / "fake.cu")] + objs, check=True)
     from dqmc_b200 import lib
     own, lib._lib = lib._lib, None

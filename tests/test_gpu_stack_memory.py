@@ -105,3 +105,34 @@ def test_clusters_stand_after_gradients(mods):
         e.close()
     for x, y in zip(*out):
         assert np.array_equal(x, y)
+
+
+def test_gradient_with_and_without_a_place_for_q(mods):
+    """the gradient's stack keeps its Q beside the clusters while half of the device
+    is free, else in their place: the same bits, and sweeps after it too"""
+    torch, engine, d = mods
+    out = []
+    for full in (False, True):
+        free, total = torch.cuda.mem_get_info()
+        hold = torch.empty(free - total // 2 + (64 << 20), dtype=torch.uint8, device="cuda") if full else None
+        s = [engine.SimData(dict(d)) for _ in range(3)]
+        for c, x in enumerate(s):
+            x.hs[:] = np.roll(x.hs, 13 * c)
+        e = engine.Engine(s)
+        e.init()
+        e.sweeps(1)
+        used0 = torch.cuda.mem_get_info()[0]
+        ld, S = e.logdet_grad()
+        took = used0 - torch.cuda.mem_get_info()[0]
+        ld2, S2 = e.logdet_grad()
+        assert np.array_equal(ld, ld2) and np.array_equal(S, S2)
+        e.sweeps(2)
+        e.pull()
+        assert e.errors() == 0
+        out.append((np.asarray(ld), np.asarray(S), s[2].hs.copy(), s[2].rng.copy(), e.g(2)[0], took))
+        e.close()
+        del hold
+        torch.cuda.empty_cache()
+    assert out[0][5] > out[1][5]                           # the place was taken only with room
+    for x, y in zip(out[0][:5], out[1][:5]):
+        assert np.array_equal(x, y)

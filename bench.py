@@ -81,16 +81,16 @@ WORKLOADS = {
 # from its accepts), with the kernel behind each
 ROOFLINE_KERNELS = {
     "gemm": "k_gemm (batched FP64 DMMA: wraps, cluster products, half wraps, UDT products)",
-    "update": "k_update (delayed rank-k Metropolis update: panel products and DMMA flush)",
-    "qr_presort": "k_qrb (pre-sorted blocked Householder QR with explicit Q, calc_eq_g)",
+    "update": "k_update_cl, k_update (delayed rank-k Metropolis update: panel products and DMMA flush)",
+    "qr_presort": "k_qrb, k_qrc (pre-sorted blocked Householder QR with explicit Q, calc_eq_g)",
     "qr_pivot": "k_qrp (column-pivoted Householder QR with explicit Q, calc_eq_g)",
-    "recombine": "k_recb (LU solve G = (D_b^-1 Q^H + D_s T)^-1 D_b^-1 Q^H)",
+    "recombine": "k_recb (LU solve of the two-sided G = Q_L D_Lb^-1 (...)^-1 D_b^-1 Q^H)",
 }
 # DRAM bytes (read + write) per chain-spin item of one launch, from ncu
 # captures of these kernels on the 12x12 model (profiles/), scaled by the
 # items of a launch; other workloads report null
-TRAFFIC_PER_ITEM = {"batch256": {"gemm": 172580, "qr_presort": 168068, "qr_pivot": 166916,
-                                 "recombine": 333636, "update": 170852}}
+TRAFFIC_PER_ITEM = {"batch256": {"gemm": 172580, "qr_presort": 167208, "qr_pivot": 166916,
+                                 "recombine": 502248, "update": 171044}}
 # the reference build's FLOPs per chain-sweep of each single-model workload,
 # counted call by call with LAPACK-standard counts (python oracle/flop_tally.py
 # after make -C oracle tally; averaged over an unequal-time cycle)

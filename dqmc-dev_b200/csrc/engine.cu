@@ -2776,10 +2776,11 @@ struct Lanes : GroupBase {
 // lanes of an engine of n_chain chains: DQMC_LANES when set, else for real
 // chains one lane per 32 from 256 chains up (at most 8) and one per 64 below
 // (at most 4), for complex chains one per 32 (at most 4).  Measured: 256
-// chains of 12 x 12 run 1235 / 1268 / 1288 / 1297 chain-sweeps/s in 2 / 4 /
-// 6 / 8 lanes (end to end 1136 in 4, 1156 in 8); the real gradients of 128
-// configurations of 8 x 8 run 719 evaluations/s in two lanes and 628 in
-// four; 64 complex 10 x 10 chains 507 in two lanes and 518 in four.
+// chains of 12 x 12 run 2072 / 2270 / 2257 / 2257 / 2249 chain-sweeps/s in 1 / 2 /
+// 4 / 6 / 8 lanes, 128 of them 2033 / 2243 / 2265 in 1 / 2 / 4; the real
+// gradients of 128 configurations of 8 x 8 take 83 / 74 / 85 ms in 1 / 2 / 4.  64
+// complex 10 x 10 chains with unequal-time measurements run 868 / 800 / 771 in 1 /
+// 2 / 4: there the rule's line is older than the kernels.
 static int lane_count(int n_chain, bool cplx)
 {
 	if (const char *v = getenv("DQMC_LANES")) {

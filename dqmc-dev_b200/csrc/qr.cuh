@@ -1318,7 +1318,8 @@ struct RecArgs {
 // Two items, N = 144: 175 us a launch (LU 183k cycles, solves 130k), against 419 us
 // for an unblocked LU with a barrier per column and solves with substitution
 // in the diagonal blocks; 512 items 0.75 ms against 1.77; N = 256 (M in L2)
-// 1.09 ms against 6.0; complex N = 100 0.50 ms for 64 items against 1.12.
+// 1.09 ms against 6.0; complex N = 100 0.27 ms for 128 items
+// against 0.59.
 
 // The magnitude a pivot is chosen by: the modulus, for complex scalars within 8%
 // of it (the octagon's norm; an infinity or a NaN stays one).  |re| + |im|, up to
@@ -1565,7 +1566,7 @@ __device__ inline void lu_u_rows(T *M, int ld, int N, int j0, int pb, int c0, in
 // M -= L U on the rows from j0 + pb on of the columns c0 .. c0+7, one warp.  A
 // complex term adds its two real products one after the other, two roundings at
 // M's size where a scalar update has one, so a complex tile sums L U by itself and
-// adds it to M once (N = 100 x 64 257 -> 265 us a launch; G of well-conditioned
+// adds it to M once (N = 100 x 128 257 -> 273 us a launch; G of well-conditioned
 // complex products 3 to 5% closer to the exact one).
 template <typename T>
 __device__ inline void lu_trail(T *M, int ld, int N, int j0, int pb, int c0, const T (&b)[2], int lane)

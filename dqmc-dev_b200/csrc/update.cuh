@@ -28,8 +28,8 @@
 // One test at a time over all of the chain's threads, two CTA-wide barriers
 // per accept (about 1700 cycles) and a row and a column of G fetched per
 // accept, took 255 us a slice at N = 144 and 68 us at N = 64 (one real chain);
-// in windows 217 and 44 us with G in device memory, where the flushes' L2
-// traffic is left, and 84 and 39 us with G on chip (update_cl.cuh), of which
+// in windows 234 and 64 us with G in device memory, where the flushes' L2
+// traffic is left, and 84 and 38 us with G on chip (update_cl.cuh), of which
 // the decisions take about 0.55 us an accept.
 //
 // The number of draws of a slice depends only on its fields at slice start

@@ -75,35 +75,37 @@ static int launch_gemm_cfg(const GemmArgs<T> &g, cudaStream_t st)
 // 3.8 / 5.6 / 9.5, x 16 8.7 / 7.1 / 9.6, x 64 21.7 / 20.7 / 16.3; complex
 // N = 100 x 2 4.8 / 8.8 / 19.3, x 32 15.4 / 18.6 / 19.4.  The lines lie where
 // the next tile overtakes: about 1000 CTAs of 16 x 16 (complex 1600), 600 of
-// 32 x 32 (real).  Beyond, the padded area counts, times what a tile takes for
-// its area (percent of a 64 tile's, gemm_tile_cost), larger tiles on ties.  The 56
-// and 40 tiles (one warp per 8 columns) are for the sizes between 64 and 48 and for
-// matrices that are at least narrow: N = 100 x 512 53 us (64: 69), N = 196 x 256 137
-// (32: 178), N = 75 x 512 31 (48: 35), complex N = 100 x 512 191 (64: 217).  A large
-// matrix of few CTAs shows their long k-steps (N = 1000 x 1: 99 us against 70 with
-// 48, complex 360 against 248), and complex 40 tiles pay from a fifth less area
-// on (N = 156 x 512 550 us against 488 with 32, N = 196 x 256 548 against 591).
-inline int gemm_tile_cost(bool cplx, int t)
+// 32 x 32 (real).  Beyond, the whole CTAs per SM count, times what a CTA of the tile
+// takes (gemm_tile_cost), larger tiles on ties: N = 100 x 512 53 us with 56 (64: 69),
+// N = 196 x 256 137 with 40 (32: 178), N = 75 x 512 31 with 40 (48: 35), complex N =
+// 100 x 512 191 with 56 (64: 217); 1000 x 1000 70 with 48 (40, the least padded area:
+// 99), complex N = 156 x 512 488 with 32 (40: 550).  Over 410 launches of 16 to 4000
+// rows the choice takes 2.7% more than the fastest tile, the least padded area 5%, with
+// 64, 48 and 32 alone 13%.
+
+// a CTA of tile t at depth K, per entry of the tile: fitted to those launches with more
+// than 900 CTAs (relative units; slope in K, and what the prologue and the stores
+// add)
+inline long long gemm_tile_cost(bool cplx, int t, int K)
 {
 	switch (t) {
-	case 56: return 108;
-	case 40: return cplx ? 120 : 102;
-	case 32: return cplx ? 100 : 103;
-	default: return 100;
+	case 64: return cplx ? 228ll * K + 3400 : 61ll * K + 2500;
+	case 56: return cplx ? 262ll * K + 3550 : 74ll * K + 1600;
+	case 48: return cplx ? 227ll * K + 3800 : 66ll * K + 1950;
+	case 40: return cplx ? 274ll * K + 1950 : 75ll * K + 1850;
+	default: return cplx ? 236ll * K + 3150 : 70ll * K + 3150;
 	}
 }
 
-inline int gemm_tile(bool cplx, int batch, int M, int N)
+inline int gemm_tile(bool cplx, int batch, int M, int N, int K)
 {
-	auto tiles = [&](int t) { return (long long)((M + t - 1) / t) * ((N + t - 1) / t); };
-	if (batch * tiles(16) <= (cplx ? 1600 : 1024)) return 16;
-	if (!cplx && batch * tiles(32) <= 600) return 32;
-	auto cost = [&](int t) { return tiles(t) * t * t * gemm_tile_cost(cplx, t); };
+	auto ctas = [&](int t) { return (long long)batch * ((M + t - 1) / t) * ((N + t - 1) / t); };
+	if (ctas(16) <= (cplx ? 1600 : 1024)) return 16;
+	if (!cplx && ctas(32) <= 600) return 32;
+	auto cost = [&](int t) { return (ctas(t) + 147) / 148 * t * t * gemm_tile_cost(cplx, t, K); };
 	int best = 64;
-	for (int t : {56, 48, 40, 32}) {
-		if ((t == 56 || t == 40) && M > 256 && N > 256) continue;
+	for (int t : {56, 48, 40, 32})
 		if (cost(t) < cost(best)) best = t;
-	}
 	return best;
 }
 
@@ -113,7 +115,7 @@ int launch_gemm(const GemmArgs<T> &g, cudaStream_t st)
 	// the scale vectors and gather indices of these modes are staged per K
 	const bool k_staged = g.mode & (GM_A_DD | GM_B_ROWD | GM_B_GATHER);
 	if ((k_staged && g.K > 512) || g.M < 1 || g.N < 1 || g.K < 1 || g.batch < 1) return DQMC_E_ARG;
-	const int best = gemm_tile(is_cplx<T>::value, g.batch, g.M, g.N);
+	const int best = gemm_tile(is_cplx<T>::value, g.batch, g.M, g.N, g.K);
 	if constexpr (is_cplx<T>::value) {
 		switch (best) {
 		case 64: return launch_gemm_cfg<T, 64, 64, 8, 4, 2, 3>(g, st);

@@ -353,7 +353,7 @@ int update_split(int N, int kd, int launch, int chains)
 	if (!pmin) return 0;
 	if (!forced) {
 		int limit;      // chains beyond which G in device memory is faster
-		if (pmin == 1) limit = CX ? (N < 56 ? chains : 110) : (N < 64 || N >= 112) ? chains : launch <= 74 ? 222 : 74;
+		if (pmin == 1) limit = CX ? (N < 56 ? 222 : 110) : (N < 64 || N >= 112) ? chains : launch <= 74 ? 222 : 74;
 		else if (pmin == 2) limit = CX && N < 112 ? 36 : 72;
 		else limit = !CX ? 60 : N < 160 ? 30 : 45;
 		if (chains > limit) return 0;
